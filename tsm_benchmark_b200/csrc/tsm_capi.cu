@@ -33,7 +33,7 @@ tsm_status cuda_fail(cudaError_t e, const char* what) {
   return TSM_ERROR_CUDA;
 }
 
-// Workspace layout: [counter u32][error u32][pad to 256 B][partials].
+// Workspace layout: [counter u32][error u32][group counters u32 x 62][partials].
 constexpr size_t kWsHeader = 256;
 constexpr int kMaxCtasPerSm = 4;
 
@@ -511,8 +511,8 @@ tsm_status tsm_fill_uniform_f64(tsm_stream_t stream, double* x, int64_t count, u
 //     (CTAs launched) * m * k * 8 B of partials.  A request that would need
 //     more returns TSM_ERROR_WORKSPACE and runs nothing.
 //   * All calls on a device share the one array and it keeps whatever the
-//     last call left.  The launch counter must start at zero, so each call
-//     zeroes it (stream-ordered) before its launch.  Calls that overlap on
+//     last call left.  The launch counters must start at zero, so each call
+//     zeroes them (stream-ordered) before its launch.  Calls that overlap on
 //     the GPU (different streams, other threads) race on the array and give
 //     wrong results: serialise them.
 //   * The first call on each device looks the array's device address up
@@ -597,7 +597,8 @@ extern "C" tsm_status tsm_gemm_tn_f64_noalloc(tsm_stream_t stream, int64_t n, in
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(p.counter, 0, sizeof(unsigned), cs);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(static scratch counter)");
+  if (e == cudaSuccess) e = cudaMemsetAsync(p.counter + 2, 0, kWsHeader - 2 * sizeof(unsigned), cs);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(static scratch counters)");
   return launch_variant(v, p, grid, cs);
 }
 

@@ -18,8 +18,9 @@
 // every cross-thread and cross-CTA sum is FP64.  Both kernels end in the same
 // deterministic two-level reduction in place of the reference's atomics: warp
 // shuffles and a fixed-order shared-memory sum give one m x k FP64 partial per
-// CTA, written to the workspace; the last CTA to finish (a counter in the
-// workspace) sums the partials in CTA order and writes C.  The result is
+// CTA, written to the workspace; groups of CTAs (counters in the workspace
+// header) sum their partials in CTA order, the last group sums the groups in
+// order and writes C.  The result is
 // bit-identical from run to run for a given variant and grid.  No value of C
 // is ever updated atomically.
 #pragma once
@@ -46,7 +47,7 @@ struct PlainArgs {
   int64_t rows_main;   // rows covered by the main loop; rows [rows_main, n) are added at the end
   int64_t num_chunks;  // bulk kernel: ceil(rows_main / RS)
   double* partials;    // workspace: gridDim.x * m * k doubles
-  unsigned* counter;   // workspace: CTAs finished in this launch (zero between launches)
+  unsigned* counter;   // workspace header: words 0 and 2.. count CTAs (zero between launches), word 1 is `error`
   unsigned* error;     // workspace: sticky error bits (dev::kErr*)
 };
 
@@ -143,7 +144,7 @@ __device__ __forceinline__ void finish_partials(const PlainArgs<T>& p, const dou
                                                 int nthreads, unsigned* s_is_last);
 
 // Sums the per-thread tiles of one CTA into `red`, then into this CTA's slot
-// of the workspace; the last CTA then writes C.  `red` must hold
+// of the workspace; the cross-CTA sum then writes C.  `red` must hold
 // slots * m * k doubles.  Called by all threads of the CTA (nthreads), of
 // which the first `cthreads` carry tiles.
 template <typename T, int EPC, int TA, int TB, int NT, bool EXACT, int WA, int WB, typename ACC>
@@ -192,11 +193,94 @@ __device__ __forceinline__ void finish_tiles(const PlainArgs<T>& p, ACC (&acc_in
   finish_partials(p, red, slots, t, nthreads, s_is_last);
 }
 
+// The sum, in order, of `count` doubles `stride` apart, sixteen loads in
+// flight; those past `count` add -0.0, which changes no sum.
+__device__ __forceinline__ double ordered_sum(const double* src, int64_t stride, int count) {
+  double s = -0.0;
+#pragma unroll 1
+  for (int b = 0; b < count; b += 16, src += 16 * stride) {
+    double v[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = b + q < count ? dev::ld_cg(src + q * stride) : -0.0;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) s += v[q];
+  }
+  return s;
+}
+
+// CTAs per group of the cross-CTA sum: one group up to 32 CTAs, ceil(sqrt(G))
+// beyond (at most 25 groups for the largest grid, 4 CTAs on each of 148 SMs).
+__device__ __forceinline__ int cta_group(int G) {
+  return G <= 32 ? G : static_cast<int>(ceilf(sqrtf(static_cast<float>(G))));
+}
+
+// Every CTA's m*k partial is in the workspace (slot blockIdx.x, written by
+// this CTA's threads just before the call).  Sums them in a fixed order, in
+// two levels: the last CTA of each group to arrive sums the group's partials
+// in CTA order into the group's first slot, and the last group to finish sums
+// the groups in order.  Calls fin(e, sum) for each entry in that one CTA;
+// skip(e) leaves an entry out.  `counter` is word 0 of the workspace header;
+// words 2.. of the header count the groups' CTAs (all zero between launches).
+//
+// Why two levels: one CTA reading all G partials is a serial tail on one SM,
+// bound by load latency (four loads in flight a thread) and, for wide C, by
+// one SM's share of L2 bandwidth: at 64 x 64 4.8 MB from 148 CTAs.  The group
+// sums run on up to 12 SMs at once with 16 loads in flight.  Up to 32 CTAs the
+// second level's fence, atomic and load cost more than they save.  B200, one
+// CTA summing -> two levels, us per call: 64 x 64 at n = 2^15 64.1 -> 32.9, at
+// 2^18 120 -> 88, at 2^21 562 -> 537; 32 x 32 at 2^15 24.4 -> 15.4; 8 x 8 at
+// 2^20 28.8 -> 26.4; 4 x 4 at 2^15 9.2 -> 7.4.
+template <typename Skip, typename Fin>
+__device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, int mk, int t, int nthreads,
+                                         unsigned* s_is_last, Skip skip, Fin fin) {
+  const int G = gridDim.x;
+  const int L = cta_group(G), NG = (G + L - 1) / L;
+  const int group = blockIdx.x / L;
+  // First the group's partials (unless there is one group), then the groups'.
+  double* src = partials + static_cast<int64_t>(group) * L * mk;
+  int64_t stride = mk;
+  int count = min(L, G - group * L);
+  unsigned* arrived = counter + 2 + group;
+  bool last_level = false;
+  if (NG == 1) {
+    arrived = counter;
+    last_level = true;
+  }
+#pragma unroll 1
+  while (true) {
+    __threadfence();
+    __syncthreads();
+    if (t == 0) {
+      const bool is_last = atomicAdd(arrived, 1u) == static_cast<unsigned>(count - 1);
+      *s_is_last = is_last ? 1u : 0u;
+      if (is_last) *arrived = 0u;  // ready for the next launch on this workspace
+    }
+    __syncthreads();
+    if (*s_is_last == 0u) return;
+    __threadfence();
+#pragma unroll 1
+    for (int e = t; e < mk; e += nthreads) {
+      if (skip(e)) continue;
+      const double s = ordered_sum(src + e, stride, count);
+      if (last_level)
+        fin(e, s);
+      else
+        src[e] = s;
+    }
+    if (last_level) return;
+    src = partials;
+    stride = static_cast<int64_t>(L) * mk;
+    count = NG;
+    arrived = counter;
+    last_level = true;
+  }
+}
+
 // Steps 3 and 4 of the reduction: the CTA's `slots` m x k FP64 partial sums
 // in `red` (shared memory, complete: the caller synchronised) are summed in
-// slot order into this CTA's workspace slot; the last CTA to arrive sums the
-// CTA partials in CTA order (plus the rows [rows_main, n) the main loop left)
-// and writes C.  Called by all `nthreads` threads of the CTA.
+// slot order into this CTA's workspace slot; then the CTAs' partials are
+// summed (sum_ctas), the rows [rows_main, n) the main loop left are added and
+// C is written.  Called by all `nthreads` threads of the CTA.
 template <typename T>
 __device__ __forceinline__ void finish_partials(const PlainArgs<T>& p, const double* red, int slots, int t,
                                                 int nthreads, unsigned* s_is_last) {
@@ -209,35 +293,26 @@ __device__ __forceinline__ void finish_partials(const PlainArgs<T>& p, const dou
     for (int q = 1; q < slots; ++q) s += red[q * mk + e];
     mine[e] = s;
   }
-  __threadfence();
-  __syncthreads();
-  if (t == 0) {
-    const unsigned prev = atomicAdd(p.counter, 1u);
-    *s_is_last = (prev == gridDim.x - 1) ? 1u : 0u;
-  }
-  __syncthreads();
-  if (*s_is_last == 0u) return;
-
-  // 4. Last CTA: partials in CTA order, then the leftover rows, then C.
-  //    Symmetric (Gram): the upper triangle is summed and written to both
+  // 4. Symmetric (Gram): the upper triangle is summed and written to both
   //    (i, j) and (j, i), so C is exactly symmetric.
-  __threadfence();
-  const int G = gridDim.x;
-  for (int e = t; e < mk; e += nthreads) {
-    const int i = e / k, j = e - (e / k) * k;
-    if (p.symmetric && i > j) continue;
-    double s = dev::ld_cg(p.partials + e);
-    for (int b = 1; b < G; ++b) s += dev::ld_cg(p.partials + static_cast<int64_t>(b) * mk + e);
-    for (int64_t r = p.rows_main; r < p.n; ++r)
-      s += static_cast<double>(p.A[r * p.lda + i]) * static_cast<double>(p.B[r * p.ldb + j]);
-    T* c = p.C + static_cast<int64_t>(i) * p.ldc + j;
-    *c = static_cast<T>(p.accumulate ? static_cast<double>(*c) + s : s);
-    if (p.symmetric && i != j) {
-      T* ct = p.C + static_cast<int64_t>(j) * p.ldc + i;
-      *ct = static_cast<T>(p.accumulate ? static_cast<double>(*ct) + s : s);
-    }
-  }
-  if (t == 0) *p.counter = 0u;  // ready for the next launch on this workspace
+  sum_ctas(
+      p.partials, p.counter, mk, t, nthreads, s_is_last,
+      [&](int e) {
+        if (!p.symmetric) return false;
+        const int i = e / k;
+        return i > e - i * k;
+      },
+      [&](int e, double s) {
+        const int i = e / k, j = e - i * k;
+        for (int64_t r = p.rows_main; r < p.n; ++r)
+          s += static_cast<double>(p.A[r * p.lda + i]) * static_cast<double>(p.B[r * p.ldb + j]);
+        T* c = p.C + static_cast<int64_t>(i) * p.ldc + j;
+        *c = static_cast<T>(p.accumulate ? static_cast<double>(*c) + s : s);
+        if (p.symmetric && i != j) {
+          T* ct = p.C + static_cast<int64_t>(j) * p.ldc + i;
+          *ct = static_cast<T>(p.accumulate ? static_cast<double>(*ct) + s : s);
+        }
+      });
 }
 
 // acc += a (TA) x b (TB) outer product.

@@ -116,32 +116,20 @@ __device__ __forceinline__ void split_finish(const SplitArgs& p, const double (&
   split_finish_ctas(p, t, nthreads, s_is_last);
 }
 
-// The CTA's partial is in the workspace (slot blockIdx.x): count the CTA in,
-// and the last one sums the CTA partials in CTA order (plus the rows
-// [rows_main, n) the pipeline left) into C.
+// The CTA's partial is in the workspace (slot blockIdx.x): the fixed-order
+// sum over CTAs (detail::sum_ctas), plus the rows [rows_main, n) the pipeline
+// left, into C.
 __device__ __forceinline__ void split_finish_ctas(const SplitArgs& p, int t, int nthreads, unsigned* s_is_last) {
   const int m = p.m, k = p.k;
-  const int mk = m * k;
-  __threadfence();
-  __syncthreads();
-  if (t == 0) {
-    const unsigned prev = atomicAdd(p.counter, 1u);
-    *s_is_last = (prev == gridDim.x - 1) ? 1u : 0u;
-  }
-  __syncthreads();
-  if (*s_is_last == 0u) return;
-  __threadfence();
-  const int64_t G = gridDim.x;
-  for (int e = t; e < mk; e += nthreads) {
-    const int i = e / k, j = e - (e / k) * k;
-    double s = dev::ld_cg(p.partials + e);
-    for (int64_t b = 1; b < G; ++b) s += dev::ld_cg(p.partials + b * mk + e);
-    for (int64_t r = p.rows_main; r < p.n; ++r)
-      s += static_cast<double>(p.A[r * m + i]) * static_cast<double>(p.B[r * k + j]);
-    double* c = p.C + static_cast<int64_t>(i) * p.ldc + j;
-    *c = p.accumulate ? *c + s : s;
-  }
-  if (t == 0) *p.counter = 0u;
+  detail::sum_ctas(
+      p.partials, p.counter, m * k, t, nthreads, s_is_last, [](int) { return false; },
+      [&](int e, double s) {
+        const int i = e / k, j = e - i * k;
+        for (int64_t r = p.rows_main; r < p.n; ++r)
+          s += static_cast<double>(p.A[r * m + i]) * static_cast<double>(p.B[r * k + j]);
+        double* c = p.C + static_cast<int64_t>(i) * p.ldc + j;
+        *c = p.accumulate ? *c + s : s;
+      });
 }
 
 __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(const SplitArgs p) {
