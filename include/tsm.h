@@ -152,10 +152,11 @@ int tsm_gemm_tn_default_variant(int dtype, int64_t n, int m, int k, const void* 
 
 typedef struct tsm_variant_info {
   char name[64];
-  int kind;    /* 0 = TMA bulk pipeline, 1 = direct loads, 2 = FP64 tensor cores (2-D TMA) */
+  int kind;    /* 0 = TMA bulk pipeline, 1 = direct loads, 2 = FP64 tensor cores (2-D TMA),
+                  3 = FP64 tensor cores, any layout and widths up to wa x wb or wb x wa */
   int dtype;   /* TSM_F64 or TSM_F32 */
   int wa, wb;  /* widths (exact) or width capacities */
-  int ta, tb;  /* per-thread tile of C (kind 2: per-warp region of C) */
+  int ta, tb;  /* per-thread tile of C (kinds 2, 3: per-warp region of C) */
   int exact;   /* 1: only m == wa, k == wb */
   int threads, stages, rows, unroll;
   size_t smem_bytes;

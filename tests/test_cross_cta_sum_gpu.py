@@ -25,7 +25,7 @@ def test_grid_sizes(gpu, oracle_mod, ctas, m, k):
                                         ws.data_ptr(), need, -1, ctas)
         assert st == 0
         got.append(C.cpu().numpy() - accumulate)
-    ref = oracle_mod.dot2(A, B) if hasattr(oracle_mod, "dot2") else oracle_mod.naive(A, B)
+    ref = oracle_mod.naive(A, B)
     for C in got:
         nw = oracle_mod.normwise(A, B, ref, C)
         assert nw["err"] <= nw["bound"], (ctas, m, k, nw)

@@ -159,7 +159,7 @@ def check(status: int, what: str = "") -> None:
     raise TsmError(status, f"{what}: {STATUS.get(status, status)}: {msg}" if what else msg)
 
 
-_KINDS = {0: "bulk", 1: "direct", 2: "dmma"}
+_KINDS = {0: "bulk", 1: "direct", 2: "dmma", 3: "direct_dmma"}
 
 
 def variants() -> list[dict]:

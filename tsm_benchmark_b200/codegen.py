@@ -297,6 +297,35 @@ class DmmaVariant:
         return f'TSM_DMMA_VARIANT("{self.name}", {v.wa}, {v.wb}, {v.mt}, {v.nt}, {v.cw}, {v.stages}, {v.rows})'
 
 
+@dataclasses.dataclass(frozen=True)
+class TileVariant:
+    """One any-layout tensor-core kernel (tsm_tn_tile_kernel,
+    csrc/tsm_tile.cuh): capacities wa >= wb, multiples of 8 up to 64, taken
+    by m x k and k x m with any strides and alignment."""
+
+    wa: int
+    wb: int
+    dtype: str = "f64"
+    exact: bool = False
+
+    @property
+    def name(self) -> str:
+        kind = "direct" if self.dtype == "f64" else "directf32"
+        return f"{kind}_dmma_{self.wa}x{self.wb}_cap"
+
+    def validate(self) -> list[str]:
+        errs = []
+        if self.wa % 8 or self.wb % 8 or not 8 <= self.wb <= self.wa <= 64:
+            errs.append("capacities must be multiples of 8, 8 <= wb <= wa <= 64")
+        if self.dtype not in ("f64", "f32"):
+            errs.append("dtype must be f64 or f32")
+        return errs
+
+    def emit(self) -> str:
+        ctype = "double" if self.dtype == "f64" else "float"
+        return f'TSM_TILE_VARIANT("{self.name}", {ctype}, {self.wa}, {self.wb})'
+
+
 DMMA_WIDTHS = (16, 32, 48, 64)
 
 
@@ -423,6 +452,11 @@ def default_variants() -> list:
     # width 32 also with 12 consumer warps.
     for w, rows, cw in ((32, 384, 8), (32, 384, 12), (48, 256, 0), (64, 192, 0), (48, 240, 12), (64, 192, 12)):
         out.append(DmmaVariant(w, w, rows=rows, stages=2, cw=cw, gram=True))
+    # Any widths, strides and alignment on the FP64 tensor cores.
+    for dtype in ("f64", "f32"):
+        for wa in range(8, 65, 8):
+            for wb in range(8, wa + 1, 8):
+                out.append(TileVariant(wa, wb, dtype))
     return out
 
 

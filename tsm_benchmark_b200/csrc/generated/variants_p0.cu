@@ -53,8 +53,17 @@ const Variant kGenPart0[] = {
     TSM_BULK_VARIANT("bulk_2x2_t2x2_w8_s6_r2048_u1_gram", double, 2, 2, 2, 2, 8, 6, 2048, 1, true, true),
     TSM_DMMA_VARIANT("dmma_16x16_t16x16_w8_s2_r384", 16, 16, 2, 2, 8, 2, 384),
     TSM_GRAM_DMMA_VARIANT("dmma_32x32_gram_w8_s2_r384", 32, 8, 2, 384),
+    TSM_TILE_VARIANT("direct_dmma_16x16_cap", double, 16, 16),
+    TSM_TILE_VARIANT("direct_dmma_40x8_cap", double, 40, 8),
+    TSM_TILE_VARIANT("direct_dmma_48x32_cap", double, 48, 32),
+    TSM_TILE_VARIANT("direct_dmma_56x48_cap", double, 56, 48),
+    TSM_TILE_VARIANT("direct_dmma_64x56_cap", double, 64, 56),
+    TSM_TILE_VARIANT("directf32_dmma_32x8_cap", float, 32, 8),
+    TSM_TILE_VARIANT("directf32_dmma_40x40_cap", float, 40, 40),
+    TSM_TILE_VARIANT("directf32_dmma_56x16_cap", float, 56, 16),
+    TSM_TILE_VARIANT("directf32_dmma_64x24_cap", float, 64, 24),
 };
 extern const int kGenPart0Count;
-const int kGenPart0Count = 46;
+const int kGenPart0Count = 55;
 
 }  // namespace tsm

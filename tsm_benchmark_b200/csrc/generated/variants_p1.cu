@@ -53,8 +53,17 @@ const Variant kGenPart1[] = {
     TSM_BULK_VARIANT("bulk_4x4_t4x4_w8_s6_r1024_u1_gram", double, 4, 4, 4, 4, 8, 6, 1024, 1, true, true),
     TSM_DMMA_VARIANT("dmma_16x16_t16x16_w8_s3_r288", 16, 16, 2, 2, 8, 3, 288),
     TSM_GRAM_DMMA_VARIANT("dmma_32x32_gram_w12_s2_r384", 32, 12, 2, 384),
+    TSM_TILE_VARIANT("direct_dmma_24x8_cap", double, 24, 8),
+    TSM_TILE_VARIANT("direct_dmma_40x16_cap", double, 40, 16),
+    TSM_TILE_VARIANT("direct_dmma_48x40_cap", double, 48, 40),
+    TSM_TILE_VARIANT("direct_dmma_56x56_cap", double, 56, 56),
+    TSM_TILE_VARIANT("direct_dmma_64x64_cap", double, 64, 64),
+    TSM_TILE_VARIANT("directf32_dmma_32x16_cap", float, 32, 16),
+    TSM_TILE_VARIANT("directf32_dmma_48x8_cap", float, 48, 8),
+    TSM_TILE_VARIANT("directf32_dmma_56x24_cap", float, 56, 24),
+    TSM_TILE_VARIANT("directf32_dmma_64x32_cap", float, 64, 32),
 };
 extern const int kGenPart1Count;
-const int kGenPart1Count = 46;
+const int kGenPart1Count = 55;
 
 }  // namespace tsm

@@ -53,8 +53,17 @@ const Variant kGenPart2[] = {
     TSM_BULK_VARIANT("bulk_8x8_t4x4_w8_s6_r512_u1_gram", double, 8, 8, 4, 4, 8, 6, 512, 1, true, true),
     TSM_GRAM_DMMA_VARIANT("dmma_16x16_gram_w8_s2_r768", 16, 8, 2, 768),
     TSM_GRAM_DMMA_VARIANT("dmma_48x48_gram_w8_s2_r256", 48, 8, 2, 256),
+    TSM_TILE_VARIANT("direct_dmma_24x16_cap", double, 24, 16),
+    TSM_TILE_VARIANT("direct_dmma_40x24_cap", double, 40, 24),
+    TSM_TILE_VARIANT("direct_dmma_48x48_cap", double, 48, 48),
+    TSM_TILE_VARIANT("direct_dmma_64x8_cap", double, 64, 8),
+    TSM_TILE_VARIANT("directf32_dmma_8x8_cap", float, 8, 8),
+    TSM_TILE_VARIANT("directf32_dmma_32x24_cap", float, 32, 24),
+    TSM_TILE_VARIANT("directf32_dmma_48x16_cap", float, 48, 16),
+    TSM_TILE_VARIANT("directf32_dmma_56x32_cap", float, 56, 32),
+    TSM_TILE_VARIANT("directf32_dmma_64x40_cap", float, 64, 40),
 };
 extern const int kGenPart2Count;
-const int kGenPart2Count = 46;
+const int kGenPart2Count = 55;
 
 }  // namespace tsm

@@ -53,8 +53,17 @@ const Variant kGenPart3[] = {
     TSM_DMMA_VARIANT("dmma_16x16_t16x16_w8_s4_r192", 16, 16, 2, 2, 8, 4, 192),
     TSM_GRAM_DMMA_VARIANT("dmma_16x16_gram_w8_s3_r512", 16, 8, 3, 512),
     TSM_GRAM_DMMA_VARIANT("dmma_64x64_gram_w8_s2_r192", 64, 8, 2, 192),
+    TSM_TILE_VARIANT("direct_dmma_24x24_cap", double, 24, 24),
+    TSM_TILE_VARIANT("direct_dmma_40x32_cap", double, 40, 32),
+    TSM_TILE_VARIANT("direct_dmma_56x8_cap", double, 56, 8),
+    TSM_TILE_VARIANT("direct_dmma_64x16_cap", double, 64, 16),
+    TSM_TILE_VARIANT("directf32_dmma_16x8_cap", float, 16, 8),
+    TSM_TILE_VARIANT("directf32_dmma_32x32_cap", float, 32, 32),
+    TSM_TILE_VARIANT("directf32_dmma_48x24_cap", float, 48, 24),
+    TSM_TILE_VARIANT("directf32_dmma_56x40_cap", float, 56, 40),
+    TSM_TILE_VARIANT("directf32_dmma_64x48_cap", float, 64, 48),
 };
 extern const int kGenPart3Count;
-const int kGenPart3Count = 46;
+const int kGenPart3Count = 55;
 
 }  // namespace tsm

@@ -53,8 +53,17 @@ const Variant kGenPart4[] = {
     TSM_DMMA_VARIANT("dmma_16x16_t16x16_w8_s6_r128", 16, 16, 2, 2, 8, 6, 128),
     TSM_DMMA_VARIANT("dmma_64x64_t32x32_w8_s2_r96", 64, 64, 4, 4, 8, 2, 96),
     TSM_GRAM_DMMA_VARIANT("dmma_48x48_gram_w12_s2_r240", 48, 12, 2, 240),
+    TSM_TILE_VARIANT("direct_dmma_32x8_cap", double, 32, 8),
+    TSM_TILE_VARIANT("direct_dmma_40x40_cap", double, 40, 40),
+    TSM_TILE_VARIANT("direct_dmma_56x16_cap", double, 56, 16),
+    TSM_TILE_VARIANT("direct_dmma_64x24_cap", double, 64, 24),
+    TSM_TILE_VARIANT("directf32_dmma_16x16_cap", float, 16, 16),
+    TSM_TILE_VARIANT("directf32_dmma_40x8_cap", float, 40, 8),
+    TSM_TILE_VARIANT("directf32_dmma_48x32_cap", float, 48, 32),
+    TSM_TILE_VARIANT("directf32_dmma_56x48_cap", float, 56, 48),
+    TSM_TILE_VARIANT("directf32_dmma_64x56_cap", float, 64, 56),
 };
 extern const int kGenPart4Count;
-const int kGenPart4Count = 46;
+const int kGenPart4Count = 55;
 
 }  // namespace tsm

@@ -53,8 +53,17 @@ const Variant kGenPart5[] = {
     TSM_DMMA_VARIANT("dmma_32x32_t32x32_w8_s4_r96", 32, 32, 4, 4, 8, 4, 96),
     TSM_DMMA_VARIANT("dmma_32x32_t32x32_w12_s2_r192", 32, 32, 4, 4, 12, 2, 192),
     TSM_GRAM_DMMA_VARIANT("dmma_64x64_gram_w12_s2_r192", 64, 12, 2, 192),
+    TSM_TILE_VARIANT("direct_dmma_32x16_cap", double, 32, 16),
+    TSM_TILE_VARIANT("direct_dmma_48x8_cap", double, 48, 8),
+    TSM_TILE_VARIANT("direct_dmma_56x24_cap", double, 56, 24),
+    TSM_TILE_VARIANT("direct_dmma_64x32_cap", double, 64, 32),
+    TSM_TILE_VARIANT("directf32_dmma_24x8_cap", float, 24, 8),
+    TSM_TILE_VARIANT("directf32_dmma_40x16_cap", float, 40, 16),
+    TSM_TILE_VARIANT("directf32_dmma_48x40_cap", float, 48, 40),
+    TSM_TILE_VARIANT("directf32_dmma_56x56_cap", float, 56, 56),
+    TSM_TILE_VARIANT("directf32_dmma_64x64_cap", float, 64, 64),
 };
 extern const int kGenPart5Count;
-const int kGenPart5Count = 46;
+const int kGenPart5Count = 55;
 
 }  // namespace tsm

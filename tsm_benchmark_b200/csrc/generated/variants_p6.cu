@@ -52,8 +52,17 @@ const Variant kGenPart6[] = {
     TSM_BULK_VARIANT("bulk_8x8_t4x4_w8_s3_r1024_u1_gram", double, 8, 8, 4, 4, 8, 3, 1024, 1, true, true),
     TSM_DMMA_VARIANT("dmma_32x32_t32x32_w8_s2_r192", 32, 32, 4, 4, 8, 2, 192),
     TSM_DMMA_VARIANT("dmma_16x16_t16x16_w12_s2_r384", 16, 16, 2, 2, 12, 2, 384),
+    TSM_TILE_VARIANT("direct_dmma_8x8_cap", double, 8, 8),
+    TSM_TILE_VARIANT("direct_dmma_32x24_cap", double, 32, 24),
+    TSM_TILE_VARIANT("direct_dmma_48x16_cap", double, 48, 16),
+    TSM_TILE_VARIANT("direct_dmma_56x32_cap", double, 56, 32),
+    TSM_TILE_VARIANT("direct_dmma_64x40_cap", double, 64, 40),
+    TSM_TILE_VARIANT("directf32_dmma_24x16_cap", float, 24, 16),
+    TSM_TILE_VARIANT("directf32_dmma_40x24_cap", float, 40, 24),
+    TSM_TILE_VARIANT("directf32_dmma_48x48_cap", float, 48, 48),
+    TSM_TILE_VARIANT("directf32_dmma_64x8_cap", float, 64, 8),
 };
 extern const int kGenPart6Count;
-const int kGenPart6Count = 45;
+const int kGenPart6Count = 54;
 
 }  // namespace tsm

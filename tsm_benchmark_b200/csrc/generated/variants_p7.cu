@@ -52,8 +52,17 @@ const Variant kGenPart7[] = {
     TSM_BULK_VARIANT("bulk_1x1_t1x1_w8_s6_r4096_u1_gram", double, 1, 1, 1, 1, 8, 6, 4096, 1, true, true),
     TSM_DMMA_VARIANT("dmma_32x32_t32x32_w8_s6_r64", 32, 32, 4, 4, 8, 6, 64),
     TSM_DMMA_VARIANT("dmma_64x64_t32x32_w12_s2_r96", 64, 64, 4, 4, 12, 2, 96),
+    TSM_TILE_VARIANT("direct_dmma_16x8_cap", double, 16, 8),
+    TSM_TILE_VARIANT("direct_dmma_32x32_cap", double, 32, 32),
+    TSM_TILE_VARIANT("direct_dmma_48x24_cap", double, 48, 24),
+    TSM_TILE_VARIANT("direct_dmma_56x40_cap", double, 56, 40),
+    TSM_TILE_VARIANT("direct_dmma_64x48_cap", double, 64, 48),
+    TSM_TILE_VARIANT("directf32_dmma_24x24_cap", float, 24, 24),
+    TSM_TILE_VARIANT("directf32_dmma_40x32_cap", float, 40, 32),
+    TSM_TILE_VARIANT("directf32_dmma_56x8_cap", float, 56, 8),
+    TSM_TILE_VARIANT("directf32_dmma_64x16_cap", float, 64, 16),
 };
 extern const int kGenPart7Count;
-const int kGenPart7Count = 45;
+const int kGenPart7Count = 54;
 
 }  // namespace tsm

@@ -15,6 +15,7 @@
 #include "../../include/tsm.h"
 #include "tsm_errors.h"
 #include "tsm_registry.cuh"
+#include "tsm_tile.h"
 #include "tsm_tmap.h"
 
 namespace tsm {
@@ -107,6 +108,7 @@ bool applicable(const Variant* v, int dtype, int64_t n, int m, int k, const void
                 int64_t ldb) {
   if (v->dtype != dtype) return false;
   if (v->gram && !is_gram(m, k, A, lda, B, ldb)) return false;
+  if (v->kind == kKindTile) return (m <= v->wa && k <= v->wb) || (m <= v->wb && k <= v->wa);
   if (v->exact ? (m != v->wa || k != v->wb) : (m > v->wa || k > v->wb)) return false;
   if (v->kind == kKindBulk) {
     if (lda != m || ldb != k) return false;
@@ -150,7 +152,67 @@ int find_variant(const char* name) {
   return -1;
 }
 
-int default_variant(int dtype, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
+int first_in_table(int dtype, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
+  const auto& vs = variants();
+  for (size_t i = 0; i < vs.size(); ++i)
+    if (vs[i]->kind != kKindTile && applicable(vs[i], dtype, n, m, k, A, lda, B, ldb)) return static_cast<int>(i);
+  return -1;
+}
+
+// The tile variant (tsm_tile.cuh) with the least capacities for m x k.
+int tile_variant(int dtype, int m, int k) {
+  static const std::vector<int> index = [] {
+    std::vector<int> v(2 * 8 * 8, -1);
+    const auto& vs = variants();
+    for (size_t i = 0; i < vs.size(); ++i)
+      if (vs[i]->kind == kKindTile)
+        v[(vs[i]->dtype * 8 + vs[i]->wa / 8 - 1) * 8 + vs[i]->wb / 8 - 1] = static_cast<int>(i);
+    return v;
+  }();
+  return index[(dtype * 8 + (std::max(m, k) - 1) / 8) * 8 + (std::min(m, k) - 1) / 8];
+}
+
+// Whether an m x k product that no variant was compiled for exactly runs on
+// the tile kernel rather than on `v`, the first capacity variant that takes
+// it: SIMT register tiles over bulk copies of contiguous rows, or over direct
+// loads.
+//
+// Contiguous rows.  The SIMT capacity kernels pad to powers of two, load one
+// element at a time and meet bank conflicts at even widths; they keep up with
+// HBM only on narrow rows, where the tile kernel's 4-row steps bound it.
+// B200, 400 MB of operands, SIMT -> tile, us: FP64 1 x 1 60 -> 152, 3 x 3
+// 63 -> 66, 8 x 1 62 -> 64, 3 x 5 67 -> 62, 5 x 5 82 -> 64, 13 x 13 87 -> 64,
+// 24 x 24 179 -> 64, 37 x 37 463 -> 85, 63 x 63 352 -> 139 (FP64-bound).
+// Below 64 MB launch and cross-CTA sum decide: 3 x 7 at n = 200001 9.4 -> 10.7,
+// 5 x 8 at 1000 5.2 -> 5.8, 13 x 13 at 1000 7.7 -> 5.4, 64 x 5 8.6 -> 6.0.
+// FP32 (the tile kernel widens to FP64, so FP64 rate bounds it): 13 x 3
+// 62 -> 84, 63 x 3 61 -> 71, 13 x 8 80 -> 69, 16 x 3 91 -> 72, 20 x 3 83 -> 82,
+// 37 x 3 92 -> 75, 24 x 24 167 -> 94, 63 x 63 252 -> 238.
+//
+// Strided or unaligned rows.  The direct kernels issue a load per element and
+// lane; tensor boxes cost by the row, so narrow slices that are loaded apart
+// stay direct: SIMT -> tile, us, 1 x 8 65 -> 112, 13 x 8 100 -> 127, 13 x 13
+// 220 -> 131, 20 x 8 142 -> 66, 40 x 1 93 -> 67.  Neighbouring slices come as
+// one: FP64 3 x 3 67 -> 71, 8 x 1 66 -> 63, 8 x 8 98 -> 63, 40 x 20 720 -> 68;
+// FP32 8 x 3 74 -> 76, 5 x 5 118 -> 82, 20 x 1 77 -> 88, 40 x 1 81 -> 74.  On a
+// thousand rows narrow ones cost the same or less direct: 3 x 5 4.8 -> 5.1,
+// FP32 5 x 8 4.8 -> 5.7; 13 x 13 7.0 -> 5.5.
+bool prefers_tile(const Variant* v, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
+  const int lo = std::min(m, k), hi = std::max(m, k);
+  const bool f64 = v->dtype == kF64;
+  const size_t e = f64 ? 8 : 4;
+  const bool small = m * k < 100 && n < (1 << 14);
+  if (is_gram(m, k, A, lda, B, ldb)) return m >= 5 && !small;  // one load for both operands
+  if (v->kind == kKindBulk)
+    return f64 ? m * k >= 100 || m + k >= 18 || (m + k >= 10 && n * (m + k) >= int64_t(1) << 23)
+               : lo >= 8 || (hi >= 16 && hi % 8 == 0) || (lo >= 3 && hi >= 20 && hi <= 48);
+  if (tile_joint(A, m, lda, B, k, ldb, e)) return !small && (f64 ? m + k >= 8 : (lo >= 3 && m * k >= 25) || hi >= 40);
+  const bool maps = aligned16(A) && aligned16(B) && lda * e % 16 == 0 && ldb * e % 16 == 0;
+  return m * k >= (maps ? 64 : 160) || m + k >= 28;
+}
+
+int default_variant(int dtype, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb,
+                    bool tiles = true) {
   const auto& vs = variants();
   // 0. C = A^T A: a Gram variant (A streamed once): the tuned entry with the
   //    largest nmin <= n for width m, else the first in table order.
@@ -189,11 +251,12 @@ int default_variant(int dtype, int64_t n, int m, int k, const void* A, int64_t l
     }
   }
   if (best >= 0) return best;
-  // 2. Table order: the generator lists exact bulk variants first, then
-  //    capacity bulk variants from the smallest capacity up, then direct ones.
-  for (size_t i = 0; i < vs.size(); ++i)
-    if (applicable(vs[i], dtype, n, m, k, A, lda, B, ldb)) return static_cast<int>(i);
-  return -1;
+  // 2. Table order: the generator lists exact variants first, then capacity
+  //    bulk variants from the smallest capacity up, then direct ones; the tile
+  //    kernel in place of a capacity one where it is faster.
+  const int idx = first_in_table(dtype, n, m, k, A, lda, B, ldb);
+  if (tiles && idx >= 0 && !vs[idx]->exact && prefers_tile(vs[idx], n, m, k, A, lda, B, ldb)) return tile_variant(dtype, m, k);
+  return idx;
 }
 
 // Rows the bulk kernels stream: every copy of rows * width elements must be a
@@ -245,6 +308,14 @@ int64_t plan_grid(const Variant* v, const DeviceState* st, int idx, PlainArgs<T>
   const int tiles = (v->wa / v->ta) * (v->wb / v->tb);
   const int64_t row_groups = v->threads / tiles;
   return std::max<int64_t>(1, std::min<int64_t>((p.n + row_groups - 1) / row_groups, max_grid));
+}
+
+template <typename T>
+void set_workspace(PlainArgs<T>& p, void* ws) {
+  unsigned char* base = static_cast<unsigned char*>(ws);
+  p.counter = reinterpret_cast<unsigned*>(base);
+  p.error = reinterpret_cast<unsigned*>(base) + 1;
+  p.partials = reinterpret_cast<double*>(base + kWsHeader);
 }
 
 template <typename T>
@@ -311,15 +382,41 @@ tsm_status launch_plain(cudaStream_t stream, int64_t n, int m, int k, const T* A
   p.ldb = ldb;
   p.ldc = ldc;
   p.accumulate = accumulate ? 1 : 0;
-  unsigned char* base = static_cast<unsigned char*>(ws);
-  p.counter = reinterpret_cast<unsigned*>(base);
-  p.error = reinterpret_cast<unsigned*>(base) + 1;
-  p.partials = reinterpret_cast<double*>(base + kWsHeader);
+  set_workspace(p, ws);
 
+  if (v->kind == kKindTile) return launch_tile<T>(v, st->sms, stream, p, lda, 1, ldb, 1, max_ctas);
   int64_t grid = plan_grid(v, st, idx, p);
   if (max_ctas > 0) grid = std::min(grid, max_ctas);  // every kernel deals its rows over any grid >= 1
   return launch_variant(v, p, grid, stream);
 }
+
+}  // namespace
+
+tsm_status run_tile_f64(cudaStream_t stream, int64_t n, int m, int k, const double* A, int64_t a_row, int64_t a_col,
+                        const double* B, int64_t b_row, int64_t b_col, double* C, int64_t ldc, int accumulate,
+                        void* ws, size_t ws_bytes) {
+  int dev = 0;
+  DeviceState* st = nullptr;
+  tsm_status s = current_device(&dev, &st);
+  if (s != TSM_SUCCESS) return s;
+  if (ws == nullptr || ws_bytes < workspace_bytes_for(st->sms, m, k) || !aligned16(ws)) return TSM_ERROR_WORKSPACE;
+  const int idx = tile_variant(kF64, m, k);
+  if (idx < 0) return TSM_ERROR_UNSUPPORTED;
+  if ((s = prepare_variant(st, idx)) != TSM_SUCCESS) return s;
+  PlainArgs<double> p{};
+  p.A = A;
+  p.B = B;
+  p.C = C;
+  p.n = n;
+  p.m = m;
+  p.k = k;
+  p.ldc = ldc;
+  p.accumulate = accumulate ? 1 : 0;
+  set_workspace(p, ws);
+  return launch_tile<double>(variants()[idx], st->sms, stream, p, a_row, a_col, b_row, b_col, 0);
+}
+
+namespace {
 
 // ------------------------------------------------------- timeout self-test
 // One thread waits on an mbarrier that nothing ever arrives on, through the
@@ -569,12 +666,6 @@ extern "C" tsm_status tsm_gemm_tn_f64_noalloc(tsm_stream_t stream, int64_t n, in
   void* scratch = nullptr;
   if ((s = static_scratch(dev, &scratch)) != TSM_SUCCESS) return s;
 
-  // Same variant and grid as tsm_gemm_tn_f64 would use.
-  const int idx = default_variant(kF64, n, m, k, A, lda, B, ldb);
-  if (idx < 0) return TSM_ERROR_UNSUPPORTED;
-  if ((s = prepare_variant(st, idx)) != TSM_SUCCESS) return s;
-  const Variant* v = variants()[idx];
-
   PlainArgs<double> p{};
   p.A = A;
   p.B = B;
@@ -586,19 +677,29 @@ extern "C" tsm_status tsm_gemm_tn_f64_noalloc(tsm_stream_t stream, int64_t n, in
   p.ldb = ldb;
   p.ldc = ldc;
   p.accumulate = accumulate ? 1 : 0;
-  const int64_t grid = plan_grid(v, st, idx, p);
-  const size_t need = kWsHeader + static_cast<size_t>(grid) * m * k * sizeof(double);
-  if (need > kStaticScratchBytes) return TSM_ERROR_WORKSPACE;
-
-  unsigned char* base = static_cast<unsigned char*>(scratch);
-  p.counter = reinterpret_cast<unsigned*>(base);
-  p.error = reinterpret_cast<unsigned*>(base) + 1;
-  p.partials = reinterpret_cast<double*>(base + kWsHeader);
+  // What the array holds is decided by the grid of the SIMT or exact variant;
+  // the tile kernel, where it takes that one's place, runs on a grid that fits.
+  int idx = default_variant(kF64, n, m, k, A, lda, B, ldb, false);
+  if (idx < 0) return TSM_ERROR_UNSUPPORTED;
+  if ((s = prepare_variant(st, idx)) != TSM_SUCCESS) return s;
+  const int64_t grid = plan_grid(variants()[idx], st, idx, p);
+  const size_t per_cta = static_cast<size_t>(m) * k * sizeof(double);
+  if (kWsHeader + static_cast<size_t>(grid) * per_cta > kStaticScratchBytes) return TSM_ERROR_WORKSPACE;
+  const int tile = default_variant(kF64, n, m, k, A, lda, B, ldb);
+  if (variants()[tile]->kind == kKindTile) {
+    idx = tile;
+    if ((s = prepare_variant(st, idx)) != TSM_SUCCESS) return s;
+  }
+  const Variant* v = variants()[idx];
+  set_workspace(p, scratch);
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(p.counter, 0, sizeof(unsigned), cs);
   if (e == cudaSuccess) e = cudaMemsetAsync(p.counter + 2, 0, kWsHeader - 2 * sizeof(unsigned), cs);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(static scratch counters)");
+  if (v->kind == kKindTile)
+    return launch_tile<double>(v, st->sms, cs, p, lda, 1, ldb, 1,
+                               static_cast<int64_t>((kStaticScratchBytes - kWsHeader) / per_cta));
   return launch_variant(v, p, grid, cs);
 }
 

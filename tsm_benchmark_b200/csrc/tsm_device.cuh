@@ -132,6 +132,21 @@ __device__ __forceinline__ uint64_t policy_evict_first() {
   return p;
 }
 
+// Asynchronous copy of one 4- or 8-byte element, global -> shared memory.
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src) {
+  static_assert(BYTES == 4 || BYTES == 8, "one element");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+
+// Arrives once on `bar` (an arrival its count includes) when every cp.async
+// this thread issued so far has landed.
+__device__ __forceinline__ void cp_async_mbar_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ double ld_shared_f64(const double* p) { return *p; }
 
 // L2-coherent load for data written by other CTAs of the same launch.

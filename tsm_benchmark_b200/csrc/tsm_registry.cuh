@@ -12,10 +12,11 @@
 
 #include "tsm_dmma.cuh"
 #include "tsm_plain.cuh"
+#include "tsm_tile.cuh"
 
 namespace tsm {
 
-enum VariantKind : int { kKindBulk = 0, kKindDirect = 1, kKindDmma = 2 };
+enum VariantKind : int { kKindBulk = 0, kKindDirect = 1, kKindDmma = 2, kKindTile = 3 };
 enum DType : int { kF64 = 0, kF32 = 1 };
 
 template <typename T>
@@ -86,4 +87,13 @@ extern const int kVariantPartCount;
     NAME, ::tsm::kKindDmma, ::tsm::kF64, W, W, 16, 16, 1, ::tsm::GramDmma<W, CW, ST, RS>::THREADS, ST, RS, 1, \
         ::tsm::GramDmma<W, CW, ST, RS>::SMEM_BYTES,                                                        \
         reinterpret_cast<const void*>(&::tsm::tsm_gram_dmma_kernel<W, CW, ST, RS>), 1                      \
+  }
+
+// Any layout on the tensor cores (tsm_tile.cuh): capacities WA >= WB, taken by
+// m x k and by k x m (rows and stages are picked at the launch).
+#define TSM_TILE_VARIANT(NAME, T, WA, WB)                                                                  \
+  ::tsm::Variant {                                                                                       \
+    NAME, ::tsm::kKindTile, ::tsm::DTypeOf<T>::value, WA, WB, 8 * ::tsm::TileKernel<WA / 8, WB / 8>::MT,     \
+        8 * ::tsm::TileKernel<WA / 8, WB / 8>::NT, 0, ::tsm::kTileThreads, ::tsm::kTileStages, 0, 1,         \
+        ::tsm::kTileSmem, reinterpret_cast<const void*>(&::tsm::tsm_tn_tile_kernel<T, WA / 8, WB / 8>), 0    \
   }
