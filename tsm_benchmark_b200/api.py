@@ -40,6 +40,38 @@ def _on_stream(device: torch.device, stream):
     return contextlib.nullcontext()  # no device: only fake allocators reach here
 
 
+_NO_GUARD = contextlib.nullcontext()
+_ws_need: dict[tuple[int, int, int], int] = {}
+
+
+def _guard(device: torch.device):
+    """Context in which `device` is current; free when it already is."""
+    return _NO_GUARD if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def _launch_on(device: torch.device, stream: torch.cuda.Stream | None, nbytes: int) -> tuple[int, torch.Tensor]:
+    """(raw stream handle, workspace of at least `nbytes` for that stream).
+    A workspace that is there already is looked up without its lock: entries
+    are only ever replaced whole."""
+    sh = torch._C._cuda_getCurrentRawStream(device.index) if stream is None else int(stream.cuda_stream)
+    ws = _workspaces.get((device.index, sh))
+    if ws is None or ws.numel() < nbytes:
+        ws = workspace(device, nbytes, _stream(device, stream))
+    return sh, ws
+
+
+def _plain_bytes(lib, device: torch.device, n: int, m: int, k: int) -> int:
+    """Workspace bytes of a plain call with these widths on `device` (current);
+    they do not depend on n."""
+    need = _ws_need.get((device.index, m, k))
+    if need is None:
+        need = lib.tsm_gemm_tn_workspace_size(n, m, k)
+        if need == 0:
+            _capi.check(1, "tsm_gemm_tn_workspace_size")
+        _ws_need[(device.index, m, k)] = need
+    return need
+
+
 def workspace(device: torch.device, nbytes: int, stream) -> torch.Tensor:
     """A zero-initialised device workspace of at least `nbytes`, one per
     (device, stream): calls on one stream are ordered, so they may share it.
@@ -67,12 +99,8 @@ def _check_operand(x: torch.Tensor, name: str, dtype: torch.dtype, any_strides: 
         raise TypeError(f"{name} must be {dtype}, got {x.dtype}")
     if x.dim() != 2:
         raise ValueError(f"{name} must be 2-D, got shape {tuple(x.shape)}")
-    if not any_strides and x.shape[0] > 0 and x.shape[1] > 1 and x.stride(1) != 1:
+    if not any_strides and x.stride(1) != 1 and x.shape[0] > 0 and x.shape[1] > 1:
         raise ValueError(f"{name} must have unit column stride (row-major rows)")
-
-
-def _row_major(x: torch.Tensor) -> bool:
-    return x.shape[0] == 0 or x.shape[1] == 1 or x.stride(1) == 1
 
 
 def _strides(x: torch.Tensor) -> tuple[int, int]:
@@ -106,43 +134,45 @@ def tsmttsm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor | None = None, *, 
     ``tsm_gemm_tn_strided_f64`` (``variant`` is then ignored).  Returns C;
     allocates it (m x k) when not given.
     """
-    if A.dtype not in _PLAIN:
-        raise TypeError(f"A must be float64 or float32, got {A.dtype}")
-    fn_name, _ = _PLAIN[A.dtype]
-    f64 = A.dtype == torch.float64
-    _check_operand(A, "A", A.dtype, any_strides=f64)
-    _check_operand(B, "B", A.dtype, any_strides=f64)
-    if A.shape[0] != B.shape[0]:
-        raise ValueError(f"A and B must have the same number of rows, got {A.shape[0]} and {B.shape[0]}")
-    if A.device != B.device:
+    dtype = A.dtype
+    if dtype not in _PLAIN:
+        raise TypeError(f"A must be float64 or float32, got {dtype}")
+    fn_name, _ = _PLAIN[dtype]
+    f64 = dtype == torch.float64
+    _check_operand(A, "A", dtype, any_strides=f64)
+    _check_operand(B, "B", dtype, any_strides=f64)
+    device = A.device
+    (n, m), (a_row, a_col) = A.shape, A.stride()
+    (nb, k), (b_row, b_col) = B.shape, B.stride()
+    if n != nb:
+        raise ValueError(f"A and B must have the same number of rows, got {n} and {nb}")
+    if device != B.device:
         raise ValueError("A and B must be on the same device")
-    n, m = A.shape
-    k = B.shape[1]
     if C is None:
         if accumulate:
             raise ValueError("accumulate=True needs an existing C")
-        C = torch.empty((m, k), dtype=A.dtype, device=A.device)
+        C = A.new_empty((m, k))
+        ldc = max(1, k)
     else:
-        _check_operand(C, "C", A.dtype)
+        _check_operand(C, "C", dtype)
         if tuple(C.shape) != (m, k):
             raise ValueError(f"C must be {m}x{k}, got {tuple(C.shape)}")
+        ldc = _ld(C)
     lib = _capi.load()
-    with torch.cuda.device(A.device):
-        so = _stream(A.device, stream)
-        sh = int(so.cuda_stream)
-        need = lib.tsm_gemm_tn_workspace_size(n, m, k)
-        if need == 0:
-            _capi.check(1, "tsm_gemm_tn_workspace_size")
-        ws = workspace(A.device, need, so)
-        if _row_major(A) and _row_major(B):
-            st = getattr(lib, fn_name)(sh, n, m, k, A.data_ptr(), _ld(A), B.data_ptr(), _ld(B), C.data_ptr(),
-                                       _ld(C), 1 if accumulate else 0, ws.data_ptr(), ws.numel(), int(variant))
-            _capi.check(st, fn_name)
+    with _guard(device):
+        sh, ws = _launch_on(device, stream, _plain_bytes(lib, device, n, m, k))
+        if (n == 0 or m == 1 or a_col == 1) and (n == 0 or k == 1 or b_col == 1):
+            lda, ldb = (max(a_row, m), max(b_row, k)) if n > 1 else (max(1, m), max(1, k))
+            st = getattr(lib, fn_name)(sh, n, m, k, A.data_ptr(), lda, B.data_ptr(), ldb, C.data_ptr(), ldc,
+                                       1 if accumulate else 0, ws.data_ptr(), ws.numel(), int(variant))
+            if st:
+                _capi.check(st, fn_name)
         else:
             (ar, ac), (br, bc) = _strides(A), _strides(B)
             st = lib.tsm_gemm_tn_strided_f64(sh, n, m, k, A.data_ptr(), ar, ac, B.data_ptr(), br, bc, C.data_ptr(),
-                                             _ld(C), 1 if accumulate else 0, ws.data_ptr(), ws.numel())
-            _capi.check(st, "tsm_gemm_tn_strided_f64")
+                                             ldc, 1 if accumulate else 0, ws.data_ptr(), ws.numel())
+            if st:
+                _capi.check(st, "tsm_gemm_tn_strided_f64")
     return C
 
 
@@ -156,19 +186,14 @@ def gram(A: torch.Tensor, C: torch.Tensor | None = None, *, accumulate: bool = F
     if C is None:
         if accumulate:
             raise ValueError("accumulate=True needs an existing C")
-        C = torch.empty((m, m), dtype=torch.float64, device=A.device)
+        C = A.new_empty((m, m))
     else:
         _check_operand(C, "C", torch.float64)
         if tuple(C.shape) != (m, m):
             raise ValueError(f"C must be {m}x{m}, got {tuple(C.shape)}")
     lib = _capi.load()
-    with torch.cuda.device(A.device):
-        so = _stream(A.device, stream)
-        sh = int(so.cuda_stream)
-        need = lib.tsm_gemm_tn_workspace_size(n, m, m)
-        if need == 0:
-            _capi.check(1, "tsm_gemm_tn_workspace_size")
-        ws = workspace(A.device, need, so)
+    with _guard(A.device):
+        sh, ws = _launch_on(A.device, stream, _plain_bytes(lib, A.device, n, m, m))
         st = lib.tsm_gram_f64(sh, n, m, A.data_ptr(), _ld(A), C.data_ptr(), _ld(C), 1 if accumulate else 0,
                               ws.data_ptr(), ws.numel())
         _capi.check(st, "tsm_gram_f64")
@@ -193,13 +218,8 @@ def block_orthogonalize(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor | None
         if tuple(C.shape) != (m, k):
             raise ValueError(f"C must be {m}x{k}, got {tuple(C.shape)}")
     lib = _capi.load()
-    with torch.cuda.device(A.device):
-        so = _stream(A.device, stream)
-        sh = int(so.cuda_stream)
-        need = lib.tsm_gemm_tn_workspace_size(n, m, k)
-        if need == 0:
-            _capi.check(1, "tsm_gemm_tn_workspace_size")
-        ws = workspace(A.device, need, so)
+    with _guard(A.device):
+        sh, ws = _launch_on(A.device, stream, _plain_bytes(lib, A.device, n, m, k))
         st = lib.tsm_block_orth_f64(sh, n, m, k, A.data_ptr(), _ld(A), B.data_ptr(), _ld(B), C.data_ptr(), _ld(C),
                                     ws.data_ptr(), ws.numel())
         _capi.check(st, "tsm_block_orth_f64")
@@ -237,7 +257,7 @@ def fill_uniform(x: torch.Tensor, seed: int, stream_id: int = 0, stream: torch.c
     if not (x.is_cuda and x.dtype == torch.float64 and x.is_contiguous()):
         raise ValueError("fill_uniform needs a contiguous float64 CUDA tensor")
     lib = _capi.load()
-    with torch.cuda.device(x.device):
+    with _guard(x.device):
         st = lib.tsm_fill_uniform_f64(_stream_handle(x.device, stream), x.data_ptr(), x.numel(),
                                       seed & 0xFFFFFFFFFFFFFFFF, stream_id & 0xFFFFFFFFFFFFFFFF)
     _capi.check(st, "tsm_fill_uniform_f64")
@@ -275,10 +295,8 @@ def tsmm(X: torch.Tensor, W: torch.Tensor, Y: torch.Tensor | None = None, *, tra
         if tuple(Y.shape) != (n, q):
             raise ValueError(f"Y must be {n}x{q}, got {tuple(Y.shape)}")
     lib = _capi.load()
-    with torch.cuda.device(X.device):
-        so = _stream(X.device, stream)
-        sh = int(so.cuda_stream)
-        ws = workspace(X.device, 256, so)
+    with _guard(X.device):
+        sh, ws = _launch_on(X.device, stream, 256)
         st = getattr(lib, _TSMM[X.dtype])(sh, n, p, q, X.data_ptr(), _ld(X), W.data_ptr(), w_row, w_col,
                                            Y.data_ptr(), _ld(Y), 1 if accumulate else 0, ws.data_ptr(), ws.numel())
         _capi.check(st, _TSMM[X.dtype])
@@ -303,10 +321,8 @@ def tsmttsm_backward(A: torch.Tensor, B: torch.Tensor, dC: torch.Tensor, *, need
     dA = torch.empty((n, m), dtype=A.dtype, device=A.device) if need_dA else None
     dB = torch.empty((n, k), dtype=A.dtype, device=A.device) if need_dB else None
     lib = _capi.load()
-    with torch.cuda.device(A.device):
-        so = _stream(A.device, stream)
-        sh = int(so.cuda_stream)
-        ws = workspace(A.device, 256, so)
+    with _guard(A.device):
+        sh, ws = _launch_on(A.device, stream, 256)
         st = getattr(lib, _BWD[A.dtype])(sh, n, m, k, A.data_ptr(), _ld(A), B.data_ptr(), _ld(B), dC.data_ptr(),
                                           k, dA.data_ptr() if dA is not None else None, m,
                                           dB.data_ptr() if dB is not None else None, k, 0, ws.data_ptr(),
@@ -341,11 +357,8 @@ def tsmttsm_split(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor | None = Non
     else:
         _check_operand(C, "C", torch.float64)
     lib = _capi.load()
-    with torch.cuda.device(A.device):
-        so = _stream(A.device, stream)
-        sh = int(so.cuda_stream)
-        need = lib.tsm_gemm_tn_workspace_size(n, m, k)
-        ws = workspace(A.device, need, so)
+    with _guard(A.device):
+        sh, ws = _launch_on(A.device, stream, lib.tsm_gemm_tn_workspace_size(n, m, k))
         if kind == "tf32":
             st = lib.tsm_gemm_tn_f32_split(sh, n, m, k, A.data_ptr(), _ld(A), B.data_ptr(), _ld(B), C.data_ptr(),
                                            _ld(C), 1 if accumulate else 0, ws.data_ptr(), ws.numel())

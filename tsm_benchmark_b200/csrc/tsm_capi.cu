@@ -152,6 +152,55 @@ int find_variant(const char* name) {
   return -1;
 }
 
+// The tuning tables, read once (every call used to scan their text and look
+// the names up: 15 us of a 25 us call): per width pair the entries by rising
+// nmin, table order for equal ones.
+struct TunedEntry {
+  long long nmin;
+  int variant;
+};
+struct TunedTables {
+  std::vector<TunedEntry> plain[65][65];
+  std::vector<TunedEntry> gram[65];
+};
+
+const TunedTables& tuned() {
+  static const TunedTables* tables = [] {
+    auto* t = new TunedTables;
+    auto add = [](std::vector<TunedEntry>& v, long long nmin, int variant) {
+      const auto at = std::upper_bound(v.begin(), v.end(), nmin,
+                                       [](long long a, const TunedEntry& e) { return a < e.nmin; });
+      v.insert(at, TunedEntry{nmin, variant});
+    };
+    for (int i = 0; i < kTunedDefaultCount; ++i) {
+      int m = 0, k = 0;
+      long long nmin = 0;
+      char name[96] = {0};
+      if (std::sscanf(kTunedDefaults[i], "%d %d %lld %95s", &m, &k, &nmin, name) != 4) continue;
+      const int idx = find_variant(name);
+      if (idx >= 0 && m >= 1 && m <= 64 && k >= 1 && k <= 64) add(t->plain[m][k], nmin, idx);
+    }
+    for (int i = 0; i < kTunedGramCount; ++i) {
+      int w = 0;
+      long long nmin = 0;
+      char name[96] = {0};
+      if (std::sscanf(kTunedGram[i], "%d %lld %95s", &w, &nmin, name) != 3) continue;
+      const int idx = find_variant(name);
+      if (idx >= 0 && w >= 1 && w <= 64 && variants()[idx]->gram) add(t->gram[w], nmin, idx);
+    }
+    return t;
+  }();
+  return *tables;
+}
+
+// The entry with the largest nmin <= n whose variant takes the request, or -1.
+int tuned_variant(const std::vector<TunedEntry>& entries, int dtype, int64_t n, int m, int k, const void* A,
+                  int64_t lda, const void* B, int64_t ldb) {
+  for (auto e = entries.rbegin(); e != entries.rend(); ++e)
+    if (e->nmin <= n && applicable(variants()[e->variant], dtype, n, m, k, A, lda, B, ldb)) return e->variant;
+  return -1;
+}
+
 int first_in_table(int dtype, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
   const auto& vs = variants();
   for (size_t i = 0; i < vs.size(); ++i)
@@ -214,42 +263,16 @@ bool prefers_tile(const Variant* v, int64_t n, int m, int k, const void* A, int6
 int default_variant(int dtype, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb,
                     bool tiles = true) {
   const auto& vs = variants();
-  // 0. C = A^T A: a Gram variant (A streamed once): the tuned entry with the
-  //    largest nmin <= n for width m, else the first in table order.
+  // 0. C = A^T A: a Gram variant (A streamed once): the tuned one, else the
+  //    first in table order.
   if (is_gram(m, k, A, lda, B, ldb)) {
-    int best = -1;
-    long long best_nmin = -1;
-    for (int i = 0; i < kTunedGramCount; ++i) {
-      int tw = 0;
-      long long nmin = 0;
-      char name[96] = {0};
-      if (std::sscanf(kTunedGram[i], "%d %lld %95s", &tw, &nmin, name) != 3) continue;
-      if (tw != m || nmin > n || nmin < best_nmin) continue;
-      const int idx = find_variant(name);
-      if (idx >= 0 && vs[idx]->gram && applicable(vs[idx], dtype, n, m, k, A, lda, B, ldb)) {
-        best = idx;
-        best_nmin = nmin;
-      }
-    }
+    const int best = tuned_variant(tuned().gram[m], dtype, n, m, k, A, lda, B, ldb);
     if (best >= 0) return best;
     for (size_t i = 0; i < vs.size(); ++i)
       if (vs[i]->gram && applicable(vs[i], dtype, n, m, k, A, lda, B, ldb)) return static_cast<int>(i);
   }
-  // 1. The tuning table: the entry with the largest nmin <= n for (m, k).
-  int best = -1;
-  long long best_nmin = -1;
-  for (int i = 0; i < kTunedDefaultCount; ++i) {
-    int tm = 0, tk = 0;
-    long long nmin = 0;
-    char name[96] = {0};
-    if (std::sscanf(kTunedDefaults[i], "%d %d %lld %95s", &tm, &tk, &nmin, name) != 4) continue;
-    if (tm != m || tk != k || nmin > n || nmin < best_nmin) continue;
-    const int idx = find_variant(name);
-    if (idx >= 0 && applicable(vs[idx], dtype, n, m, k, A, lda, B, ldb)) {
-      best = idx;
-      best_nmin = nmin;
-    }
-  }
+  // 1. The tuning table.
+  const int best = tuned_variant(tuned().plain[m][k], dtype, n, m, k, A, lda, B, ldb);
   if (best >= 0) return best;
   // 2. Table order: the generator lists exact variants first, then capacity
   //    bulk variants from the smallest capacity up, then direct ones; the tile
