@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tsm_tn_tile_kernel(const __gr
   using K = TileKernel<TA, TB>;
   constexpr int CW = kTileConsumers, STAGES = kTileStages;
   const PlainArgs<T>& p = args.p;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((128u - (dev::smem_u32(smem_raw) & 127u)) & 127u);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kTileData);
   uint64_t* empty = full + STAGES;
@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tsm_tn_tile_kernel(const __gr
         atomicOr(p.error, dev::kErrTimeout);
         break;
       }
+      __syncwarp();
       const unsigned char* stage = smem + s * args.stage_bytes;
       const T* sa = reinterpret_cast<const T*>(stage + xa.offset) + xa.first + base_a;
       const T* sb = reinterpret_cast<const T*>(stage + xb.offset) + xb.first + base_b;
@@ -334,7 +335,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) tsm_tn_tile_kernel(const __gr
           }
         }
       } else {
-        // the last chunk: rows past the end contribute zeros
+        // The last chunk: rows past the end contribute zeros.  They are read (the
+        // stage holds them) and replaced with a select: no lane may branch
+        // around a load here, or the warp could reach the warp-wide MMAs in
+        // two parts, which never end.
         const int rows = static_cast<int>(left);
 #pragma unroll 1
         for (int ks = slot; ks < ksteps; ks += K::S) {
@@ -345,9 +349,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) tsm_tn_tile_kernel(const __gr
           const T* yb = at_b(ks);
           double a[K::MT], b[K::NT];
 #pragma unroll
-          for (int i = 0; i < K::MT; ++i) a[i] = in ? static_cast<double>(ya[8 * i]) : 0.0;
+          for (int i = 0; i < K::MT; ++i) {
+            const double v = static_cast<double>(ya[8 * i]);
+            a[i] = in ? v : 0.0;
+          }
 #pragma unroll
-          for (int j = 0; j < K::NT; ++j) b[j] = in ? static_cast<double>(yb[8 * j]) : 0.0;
+          for (int j = 0; j < K::NT; ++j) {
+            const double v = static_cast<double>(yb[8 * j]);
+            b[j] = in ? v : 0.0;
+          }
+          __syncwarp();
           mma(acc[0], a, b);
         }
       }
