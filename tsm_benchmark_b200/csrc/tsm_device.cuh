@@ -101,6 +101,23 @@ __device__ __forceinline__ void bulk_g2s_evict_first(void* dst, const void* src,
       : "memory");
 }
 
+// 1-D bulk copy shared -> global memory, part of the issuing thread's current
+// bulk group.  Both addresses and bytes must be multiples of 16; generic writes
+// to the source need fence_proxy_async_smem() before it.
+__device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t bytes, uint64_t policy) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(dst),
+               "r"(smem_u32(src)), "r"(bytes), "l"(policy)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Until at most N of this thread's bulk groups still read shared memory.
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+// Until all of this thread's bulk groups are complete.
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // 2-D tiled TMA load, into this CTA alone, of the box at element coordinates
 // (x, y) of `tmap` into this CTA's shared memory, completing the box's bytes
 // on `bar`.  x * element size must be a multiple of 16 bytes; rows y beyond

@@ -12,6 +12,7 @@
 #include "tsm_errors.h"
 #include "tsm_tsmm.cuh"
 #include "tsm_tsmm_dmma.cuh"
+#include "tsm_tsmm_tile.cuh"
 
 namespace tsm {
 namespace {
@@ -203,11 +204,115 @@ tsm_status launch_dmma(cudaStream_t stream, int dev, int sms, const TsmmProblem<
     if (a.total_chunks == 0 && a.prob[0].n == 0 && (a.nprob < 2 || a.prob[1].n == 0)) continue;
     const int64_t grid =
         std::max<int64_t>(1, std::min<int64_t>(a.total_chunks, int64_t(sms) * g_dmma_ctas[dev][idx[l]]));
+    // In turn only on an even grid: a CTA then keeps to one problem and loads its W once.
+    a.alternate = a.nprob == 2 && a.prob[0].num_chunks == a.prob[1].num_chunks && grid % 2 == 0;
     void* args[] = {&a};
     const cudaError_t le =
         cudaLaunchKernel(e.fn, dim3(static_cast<unsigned>(grid)), dim3(e.threads), args, e.smem, stream);
     if (le != cudaSuccess) return fail(le, "cudaLaunchKernel(tsmm dmma)");
   }
+  return TSM_SUCCESS;
+}
+
+signed char g_tile_ready[64][2] = {};
+
+int round128(int x) { return (x + 127) / 128 * 128; }
+
+// The tile kernel takes X and Y dense and 16-byte aligned.
+template <typename T>
+bool tile_takes(const TsmmProblem<T>& pr) {
+  return pr.ldx == pr.p && pr.ldy == pr.q && aligned16(pr.X) && aligned16(pr.Y);
+}
+
+// Whether dense problems run on the tile kernel rather than on the kernels for
+// powers of two (tsm_tsmm_dmma.cuh), which keep W in registers.
+//
+// B200, dmma -> tile, us.  Backward (both products), ~400 MB: FP64 13 x 13
+// 118 -> 67, 24 x 24 139 -> 74, 37 x 13 170 -> 75, 48 x 48 219 -> 112, 63 x 63
+// 169 -> 138, 5 x 8 68 -> 67; FP32 24 x 24 269 -> 112, 63 x 63 327 -> 231.
+// Powers of two, backward: FP64 16 x 16 65 -> 67, 32 x 32 158 -> 178 (500 MB),
+// 64 x 64 113 -> 124, FP32 8 x 8 69 -> 88; on few rows the finer chunks win at
+// 32 and 64, and unequal widths are two launches there: 3 MB of operands, FP64
+// 32 x 32 6.5 -> 6.0, 8 x 32 9.0 -> 5.1, 64 x 16 13.3 -> 5.8, FP32 32 x 32 16.6
+// -> 6.9; 20 MB, FP64 32 x 32 12.5 -> 12.8, 64 x 16 16.2 -> 13.1, FP32 32 x 32
+// 24.9 -> 19.1, 4 x 8 11.7 -> 14.3.  Y += X W: 16 x 16 26.7 -> 27.8 (20 MB),
+// 33.9 -> 38.5 (100 MB).
+template <typename T>
+bool prefers_tile(const TsmmProblem<T>* probs, int nprob) {
+  bool pow2 = true, equal = true, beta = true;
+  int64_t bytes = 0;  // read and written
+  int lo = 64, hi = 0;
+  for (int i = 0; i < nprob; ++i) {
+    const TsmmProblem<T>& pr = probs[i];
+    if (!tile_takes(pr)) return false;
+    pow2 = pow2 && std::min(pr.p, pr.q) >= 4 && (pr.p & (pr.p - 1)) == 0 && (pr.q & (pr.q - 1)) == 0;
+    lo = std::min(lo, std::min(pr.p, pr.q));
+    hi = std::max(hi, std::max(pr.p, pr.q));
+    equal = equal && pr.p == pr.q;
+    beta = beta && pr.beta;
+    bytes += pr.n * (pr.p + pr.q) * int64_t(sizeof(T));
+  }
+  const bool f64 = sizeof(T) == 8;
+  if (!pow2) return !(f64 && lo > 56 && bytes < (int64_t(16) << 20));
+  if (beta || nprob == 1) return false;
+  const bool small = bytes < (int64_t(12) << 20), medium = bytes < (int64_t(48) << 20);
+  if (equal) return f64 ? hi == 32 && small : hi >= 32 && medium;
+  return small || (medium && (f64 ? hi == 64 : hi >= 32));
+}
+
+template <typename T>
+tsm_status launch_tile(cudaStream_t stream, int dev, int sms, const TsmmProblem<T>* probs, int nprob,
+                       unsigned* error) {
+  const void* fn = reinterpret_cast<const void*>(&tsm_tsmm_tile_kernel<T>);
+  {
+    std::lock_guard<std::mutex> lk(g_tsmm_mu);
+    signed char& ready = g_tile_ready[dev][sizeof(T) == 8 ? 0 : 1];
+    if (!ready) {
+      const cudaError_t ce =
+          cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTsmmTileSmem));
+      if (ce != cudaSuccess) return fail(ce, "cudaFuncSetAttribute(tsmm tile)");
+      ready = 1;
+    }
+  }
+  TsmmTileArgs<T> args{};
+  TsmmArgs<T>& a = args.a;
+  a.error = error;
+  a.nprob = nprob;
+  int64_t most_rows = 0;
+  int row_elems = 0, off = 0;
+  for (int i = 0; i < nprob; ++i) {
+    a.prob[i] = probs[i];
+    TsmmProblem<T>& pr = a.prob[i];
+    pr.rows_main = std::min(tsmm_bulk_rows(pr.n, pr.p, sizeof(T)), tsmm_bulk_rows(pr.n, pr.q, sizeof(T)));
+    most_rows = std::max(most_rows, pr.rows_main);
+    row_elems = std::max(row_elems, pr.p + pr.q);
+    args.w_offset[i] = off;
+    off += tsmm_ksteps(pr.p) * tsmm_tiles(pr.q) * 32 * int(sizeof(double));
+  }
+  args.ring = round128(off);
+  // Chunk: what the stages hold, whole 32-row units, at most 2048 rows; fewer
+  // where the rows would not fill the grid evenly.
+  const int slack = 128 + 256;  // rounding of the X part, reads past its last row
+  const int budget = (int(kTsmmTileData) - args.ring) / kTsmmTileStages / 128 * 128 - slack;
+  const int most = std::min(2048, budget / (row_elems * int(sizeof(T)))) / 32 * 32;
+  const int64_t waves = std::max<int64_t>(1, (most_rows * nprob + int64_t(sms) * most - 1) / (int64_t(sms) * most));
+  const int64_t even = (most_rows * nprob + sms * waves - 1) / (sms * waves);
+  args.rs = static_cast<int>(std::min<int64_t>(most, std::max<int64_t>(32, (even + 31) / 32 * 32)));
+  for (int i = 0; i < nprob; ++i) {
+    TsmmProblem<T>& pr = a.prob[i];
+    pr.num_chunks = (pr.rows_main + args.rs - 1) / args.rs;
+    a.total_chunks += pr.num_chunks;
+    args.y_offset[i] = round128(args.rs * pr.p * int(sizeof(T)) + 64);
+    args.stage_bytes = std::max(args.stage_bytes, round128(args.y_offset[i] + args.rs * pr.q * int(sizeof(T))));
+  }
+  a.split = a.prob[0].num_chunks;
+  a.alternate = nprob == 2 && a.prob[0].num_chunks == a.prob[1].num_chunks;
+  if (a.prob[0].n == 0 && (nprob < 2 || a.prob[1].n == 0)) return TSM_SUCCESS;
+  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(a.total_chunks, sms));
+  void* params[] = {&args};
+  const cudaError_t le = cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(kTsmmTileThreads), params,
+                                          kTsmmTileSmem, stream);
+  if (le != cudaSuccess) return fail(le, "cudaLaunchKernel(tsmm tile)");
   return TSM_SUCCESS;
 }
 
@@ -237,6 +342,7 @@ tsm_status launch_tsmm(cudaStream_t stream, TsmmProblem<T>* probs, int nprob, vo
     }
   }
   const int sms = g_sms[dev];
+  if (bulk && prefers_tile(probs, nprob)) return launch_tile<T>(stream, dev, sms, probs, nprob, reinterpret_cast<unsigned*>(ws) + 1);
   if (bulk) return launch_dmma<T>(stream, dev, sms, probs, nprob, reinterpret_cast<unsigned*>(ws) + 1);
 
   int idx = -1;

@@ -7,7 +7,8 @@
 // between the two problems.
 //
 // Kernels: dense, 16-byte aligned X streams through a TMA ring into the FP64
-// tensor cores (tsm_tsmm_dmma.cuh); any other X (a column slice, an odd
+// tensor cores (tsm_tsmm_dmma.cuh; tsm_tsmm_tile.cuh for widths that are not
+// powers of two and dense Y); any other X (a column slice, an odd
 // row stride) takes the SIMT kernel below, which loads rows directly:
 //   * each lane owns ONE output column o of Y and keeps column o of W in
 //     registers (C = capacity of p and q, a power of two <= 64);
@@ -49,10 +50,30 @@ struct TsmmArgs {
   int nprob;
   int64_t split;  // chunks [0, split) belong to prob[0], the rest to prob[1]
   int64_t total_chunks;
+  int alternate;  // 1: both problems have the same number of chunks, taken in turn
   unsigned* error;
 };
 
 namespace detail {
+
+// Which problem the c-th chunk taken belongs to, and its first row (chunks of
+// `rs` rows).  Chunks are taken from the last rows to the first, those of two
+// problems in turn: the product before this one (A^T B in the forward pass or
+// in block orthogonalisation) read A and B in rising row order, and its last
+// reads are what L2 still holds.  B200, rising -> falling order, us: forward and
+// backward of 2^22 x 16 x 16 FP32 264 -> 258, FP64 507 -> 497, of 2^20 x 8 x 8
+// 77 -> 68; block orthogonalisation of 2^20 rows, m = 32, k = 8, 112 -> 100.
+template <typename T>
+__device__ __forceinline__ void tsmm_chunk(const TsmmArgs<T>& a, int64_t c, int rs, int& pi, int64_t& r0) {
+  const int64_t back = a.total_chunks - 1 - c;
+  if (a.alternate) {
+    pi = static_cast<int>(back & 1);
+    r0 = (back >> 1) * rs;
+  } else {
+    pi = back < a.split ? 0 : 1;
+    r0 = (back - (pi ? a.split : 0)) * rs;
+  }
+}
 
 template <typename T, int C>
 __device__ __forceinline__ void load_w_column(const TsmmProblem<T>& pr, int o, T (&w)[C]) {

@@ -180,9 +180,10 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
       if (lane == 0) {
         if (round > 0) ok = dev::mbar_wait(&empty[s], static_cast<uint32_t>((round - 1) & 1), abort);
         if (ok) {
-          const int pi = c < args.split ? 0 : 1;
+          int pi;
+          int64_t r0;
+          detail::tsmm_chunk(args, c, RS, pi, r0);
           const TsmmProblem<TX>& pr = args.prob[pi];
-          const int64_t r0 = (c - (pi ? args.split : 0)) * RS;
           const int64_t rows = (pr.rows_main - r0) < RS ? (pr.rows_main - r0) : RS;
           const uint32_t bytes = static_cast<uint32_t>(rows * pr.p * sizeof(TX));
           const uint32_t ybytes = YS ? static_cast<uint32_t>(rows * pr.q * sizeof(TX)) : 0u;
@@ -210,7 +211,9 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
     int64_t it = 0;
     for (int64_t c = blockIdx.x; c < args.total_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      const int pi = c < args.split ? 0 : 1;
+      int pi;
+      int64_t r0;
+      detail::tsmm_chunk(args, c, RS, pi, r0);
       const TsmmProblem<TX>& pr = args.prob[pi];
       if (pi != cur) {
         detail::load_w_frags<TX, K::KS, K::NT>(pr, o0, g, t, b);
@@ -221,7 +224,6 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
         atomicOr(args.error, dev::kErrTimeout);
         break;
       }
-      const int64_t r0 = (c - (pi ? args.split : 0)) * RS;
       const int rows = static_cast<int>((pr.rows_main - r0) < RS ? (pr.rows_main - r0) : RS);
       const TX* stage = ring + s * K::STAGE_ALL;
       const TX* ystage = stage + K::STAGE;  // old Y rows, pitch q (YS only)
