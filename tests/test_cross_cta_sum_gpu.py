@@ -1,5 +1,5 @@
-"""The cross-CTA sum at the edges of its two levels: one group up to 32 CTAs,
-groups of ceil(sqrt(G)) beyond, odd and even m*k, a ragged last group."""
+"""The cross-CTA sum at the edges of its two levels: one group up to 32 CTAs
+(64 where m*k <= 256), groups of ceil(sqrt(G)) beyond, odd and even m*k, a ragged last group."""
 import numpy as np
 import pytest
 import torch
@@ -7,7 +7,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("ctas", [1, 2, 16, 17, 31, 32, 33, 37, 144, 145, 148])
+@pytest.mark.parametrize("ctas", [1, 2, 16, 17, 31, 32, 33, 37, 64, 65, 144, 145, 148])
 @pytest.mark.parametrize("m,k", [(3, 5), (8, 8), (64, 64)])
 def test_grid_sizes(gpu, oracle_mod, ctas, m, k):
     from tsm_benchmark_b200 import _capi

@@ -7,7 +7,7 @@
     python -m tsm_benchmark_b200.autotune --shapes gram              (the Gram variant per width, C = A^T A)
 
 For every width pair and row bucket it times each applicable variant of the
-table (CUDA events, warm-up then repeated launches, inputs larger than L2
+table (CUDA events around graphs of repeated launches, inputs larger than L2
 where the bucket allows), checks every candidate against the first one's
 result (the checksum identity and a normwise bound), re-times the best
 three (those within 5 % of the fastest) in interleaved rounds and records
@@ -39,7 +39,7 @@ GRAM_WIDTHS = [1, 2, 4, 8, 16, 32, 48, 64]
 KEPT_SECTIONS = ("batched_paths", "gram_choices", "gram_timings")
 BATCHED_PAIRS = [(a, b) for a in (4, 8, 16, 32) for b in (4, 8, 16, 32)]
 # (nmin, n to time at): the largest nmin <= n selects the entry at run time.
-BUCKETS = [(0, 1 << 15), (1 << 18, 1 << 20), (1 << 23, 1 << 26)]
+BUCKETS = [(0, 1 << 12), (1 << 14, 1 << 16), (1 << 18, 1 << 20), (1 << 23, 1 << 26)]
 MAX_BYTES = 24 << 30  # per operand pair while tuning
 
 
@@ -53,14 +53,18 @@ def _cap(w: int) -> int:
 def candidates(variants: list[dict], m: int, k: int, dtype: str = "f64") -> list[dict]:
     """Variants of `dtype` that accept (m, k) for distinct A and B: every
     exact one, and the capacity ones no more than twice the smallest capacity
-    per side (larger ones only add masked work).  Gram variants (B is A)
-    are not candidates."""
+    per side (larger ones only add masked work); of the any-layout
+    tensor-core ones only the one with the least capacities.  Gram variants
+    (B is A) are not candidates."""
     out = []
     cm, ck = _cap(m), _cap(k)
     for v in variants:
         if v["dtype"] != dtype or v.get("gram"):
             continue
-        if v["exact"]:
+        if v["kind"] == "direct_dmma":
+            if (v["wa"], v["wb"]) == (-(-m // 8) * 8, -(-k // 8) * 8):
+                out.append(v)
+        elif v["exact"]:
             if m == v["wa"] and k == v["wb"]:
                 out.append(v)
         elif m <= v["wa"] <= 2 * cm and k <= v["wb"] <= 2 * ck:
@@ -117,17 +121,42 @@ def merge_results(old: dict, res: dict, pairs) -> dict:
 
 
 def time_variant(call, reps: int, warmup: int = 3) -> float:
+    """Milliseconds a call, over `reps` of them captured in CUDA graphs: a
+    call launched from Python takes 10 us of host time, more than a kernel on
+    few rows, and would hide what the tuner compares."""
     import torch
-    for _ in range(warmup):
-        call()
-    e0 = torch.cuda.Event(enable_timing=True)
-    e1 = torch.cuda.Event(enable_timing=True)
-    e0.record()
-    for _ in range(reps):
-        call()
-    e1.record()
-    torch.cuda.synchronize()
-    return e0.elapsed_time(e1) / reps
+    side = _capture_stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(warmup):
+            call()
+        graph = torch.cuda.CUDAGraph()
+        per = min(reps, 50)
+        with torch.cuda.graph(graph, stream=side):
+            for _ in range(per):
+                call()
+        rounds = max(1, reps // per)
+        e0 = torch.cuda.Event(enable_timing=True)
+        e1 = torch.cuda.Event(enable_timing=True)
+        graph.replay()
+        e0.record(side)
+        for _ in range(rounds):
+            graph.replay()
+        e1.record(side)
+        side.synchronize()
+    torch.cuda.current_stream().wait_stream(side)
+    return e0.elapsed_time(e1) / (rounds * per)
+
+
+_side = None
+
+
+def _capture_stream():
+    global _side
+    import torch
+    if _side is None:
+        _side = torch.cuda.Stream()
+    return _side
 
 
 def refine(row: dict, make_call, nbytes: int, reps_time_ms: float, rounds: int):

@@ -195,9 +195,9 @@ const TunedTables& tuned() {
 
 // The entry with the largest nmin <= n whose variant takes the request, or -1.
 int tuned_variant(const std::vector<TunedEntry>& entries, int dtype, int64_t n, int m, int k, const void* A,
-                  int64_t lda, const void* B, int64_t ldb) {
+                  int64_t lda, const void* B, int64_t ldb, bool tiles = true) {
   for (auto e = entries.rbegin(); e != entries.rend(); ++e)
-    if (e->nmin <= n && applicable(variants()[e->variant], dtype, n, m, k, A, lda, B, ldb)) return e->variant;
+    if (e->nmin <= n && (tiles || variants()[e->variant]->kind != kKindTile) && applicable(variants()[e->variant], dtype, n, m, k, A, lda, B, ldb)) return e->variant;
   return -1;
 }
 
@@ -221,10 +221,16 @@ int tile_variant(int dtype, int m, int k) {
   return index[(dtype * 8 + (std::max(m, k) - 1) / 8) * 8 + (std::min(m, k) - 1) / 8];
 }
 
-// Whether an m x k product that no variant was compiled for exactly runs on
-// the tile kernel rather than on `v`, the first capacity variant that takes
-// it: SIMT register tiles over bulk copies of contiguous rows, or over direct
-// loads.
+// Whether an m x k product that has no tuned entry runs on the tile kernel
+// rather than on `v`, the first variant in the table that takes it.
+//
+// FP32 squares compiled exactly stay, but for few rows of wide ones, where
+// their long chunks leave SMs idle: SIMT -> tile, us, 16 x 16 at n = 1000 9.2 ->
+// 5.8, at 2^18 15.4 -> 13.5, at 2^20 28.3 -> 30.7; 32 x 32 at 2^16 19.9 -> 17.1;
+// 64 x 64 at 2^16 49.6 -> 41.9, at 2^20 254 -> 293; 8 x 8 at 2^18 9.5 -> 11.0.
+//
+// The rest run on SIMT register tiles of a larger capacity, over bulk copies of
+// contiguous rows or over direct loads.
 //
 // Contiguous rows.  The SIMT capacity kernels pad to powers of two, load one
 // element at a time and meet bank conflicts at even widths; they keep up with
@@ -250,6 +256,7 @@ bool prefers_tile(const Variant* v, int64_t n, int m, int k, const void* A, int6
   const int lo = std::min(m, k), hi = std::max(m, k);
   const bool f64 = v->dtype == kF64;
   const size_t e = f64 ? 8 : 4;
+  if (v->exact) return !f64 && v->kind == kKindBulk && lo >= 16 && n * (m + k) <= int64_t(1) << 23;
   const bool small = m * k < 100 && n < (1 << 14);
   if (is_gram(m, k, A, lda, B, ldb)) return m >= 5 && !small;  // one load for both operands
   if (v->kind == kKindBulk)
@@ -272,13 +279,13 @@ int default_variant(int dtype, int64_t n, int m, int k, const void* A, int64_t l
       if (vs[i]->gram && applicable(vs[i], dtype, n, m, k, A, lda, B, ldb)) return static_cast<int>(i);
   }
   // 1. The tuning table.
-  const int best = tuned_variant(tuned().plain[m][k], dtype, n, m, k, A, lda, B, ldb);
+  const int best = tuned_variant(tuned().plain[m][k], dtype, n, m, k, A, lda, B, ldb, tiles);
   if (best >= 0) return best;
   // 2. Table order: the generator lists exact variants first, then capacity
   //    bulk variants from the smallest capacity up, then direct ones; the tile
   //    kernel in place of a capacity one where it is faster.
   const int idx = first_in_table(dtype, n, m, k, A, lda, B, ldb);
-  if (tiles && idx >= 0 && !vs[idx]->exact && prefers_tile(vs[idx], n, m, k, A, lda, B, ldb)) return tile_variant(dtype, m, k);
+  if (tiles && idx >= 0 && prefers_tile(vs[idx], n, m, k, A, lda, B, ldb)) return tile_variant(dtype, m, k);
   return idx;
 }
 

@@ -208,10 +208,11 @@ __device__ __forceinline__ double ordered_sum(const double* src, int64_t stride,
   return s;
 }
 
-// CTAs per group of the cross-CTA sum: one group up to 32 CTAs, ceil(sqrt(G))
-// beyond (at most 25 groups for the largest grid, 4 CTAs on each of 148 SMs).
-__device__ __forceinline__ int cta_group(int G) {
-  return G <= 32 ? G : static_cast<int>(ceilf(sqrtf(static_cast<float>(G))));
+// CTAs per group of the cross-CTA sum: one group up to 32 CTAs (64 where C is
+// small), ceil(sqrt(G)) beyond (at most 25 groups for the largest grid, 4 CTAs
+// on each of 148 SMs).
+__device__ __forceinline__ int cta_group(int G, int mk) {
+  return G <= 32 || (G <= 64 && mk <= 256) ? G : static_cast<int>(ceilf(sqrtf(static_cast<float>(G))));
 }
 
 // Every CTA's m*k partial is in the workspace (slot blockIdx.x, written by
@@ -225,8 +226,9 @@ __device__ __forceinline__ int cta_group(int G) {
 // Why two levels: one CTA reading all G partials is a serial tail on one SM,
 // bound by load latency (four loads in flight a thread) and, for wide C, by
 // one SM's share of L2 bandwidth: at 64 x 64 4.8 MB from 148 CTAs.  The group
-// sums run on up to 12 SMs at once with 16 loads in flight.  Up to 32 CTAs the
-// second level's fence, atomic and load cost more than they save.  B200, one
+// sums run on up to 12 SMs at once with 16 loads in flight.  On few CTAs the
+// second level's fence, atomic and load cost more than they save (4 x 4 Gram
+// at n = 10^5, 49 CTAs: 8.5 us with two levels, 7.1 with one).  B200, one
 // CTA summing -> two levels, us per call: 64 x 64 at n = 2^15 64.1 -> 32.9, at
 // 2^18 120 -> 88, at 2^21 562 -> 537; 32 x 32 at 2^15 24.4 -> 15.4; 8 x 8 at
 // 2^20 28.8 -> 26.4; 4 x 4 at 2^15 9.2 -> 7.4.
@@ -234,7 +236,7 @@ template <typename Skip, typename Fin>
 __device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, int mk, int t, int nthreads,
                                          unsigned* s_is_last, Skip skip, Fin fin) {
   const int G = gridDim.x;
-  const int L = cta_group(G), NG = (G + L - 1) / L;
+  const int L = cta_group(G, mk), NG = (G + L - 1) / L;
   const int group = blockIdx.x / L;
   // First the group's partials (unless there is one group), then the groups'.
   double* src = partials + static_cast<int64_t>(group) * L * mk;
