@@ -41,7 +41,7 @@ Layout layout(int count, int nseg, int grid, size_t partial_doubles) {
   l.cta_first = off;
   off = align_up(off + sizeof(int) * (grid + 1));
   l.counters = off;
-  off = align_up(off + sizeof(unsigned) * count);
+  off = align_up(off + sizeof(unsigned) * batched::kCountersPerProblem * count);
   l.partials = off;
   off = align_up(off + sizeof(double) * partial_doubles);
   l.total = off;

@@ -215,13 +215,16 @@ __device__ __forceinline__ int cta_group(int G, int mk) {
   return G <= 32 || (G <= 64 && mk <= 256) ? G : static_cast<int>(ceilf(sqrtf(static_cast<float>(G))));
 }
 
-// Every CTA's m*k partial is in the workspace (slot blockIdx.x, written by
-// this CTA's threads just before the call).  Sums them in a fixed order, in
-// two levels: the last CTA of each group to arrive sums the group's partials
-// in CTA order into the group's first slot, and the last group to finish sums
-// the groups in order.  Calls fin(e, sum) for each entry in that one CTA;
-// skip(e) leaves an entry out.  `counter` is word 0 of the workspace header;
-// words 2.. of the header count the groups' CTAs (all zero between launches).
+// `G` members' m*k partials lie one after another, each written by its member's
+// threads just before the call (this one is `member`; a member is a CTA, or a
+// segment of a batched problem, and `sync` its threads' barrier).  Sums them in a
+// fixed order, in
+// two levels: the last member of each group to arrive sums the group's partials
+// in order into the group's first slot, and the last group to finish sums
+// the groups in order.  Calls fin(e, sum) for each entry in that one member;
+// skip(e) leaves an entry out.  `counter` and the words from
+// counter + 2 on, one per group, count arrivals (all zero between launches; in
+// a workspace header word 1 is the error word).
 //
 // Why two levels: one CTA reading all G partials is a serial tail on one SM,
 // bound by load latency (four loads in flight a thread) and, for wide C, by
@@ -232,12 +235,11 @@ __device__ __forceinline__ int cta_group(int G, int mk) {
 // CTA summing -> two levels, us per call: 64 x 64 at n = 2^15 64.1 -> 32.9, at
 // 2^18 120 -> 88, at 2^21 562 -> 537; 32 x 32 at 2^15 24.4 -> 15.4; 8 x 8 at
 // 2^20 28.8 -> 26.4; 4 x 4 at 2^15 9.2 -> 7.4.
-template <typename Skip, typename Fin>
-__device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, int mk, int t, int nthreads,
-                                         unsigned* s_is_last, Skip skip, Fin fin) {
-  const int G = gridDim.x;
+template <typename Sync, typename Skip, typename Fin>
+__device__ __forceinline__ void sum_members(double* partials, unsigned* counter, int G, int member, int mk, int t,
+                                            int nthreads, unsigned* s_is_last, Sync sync, Skip skip, Fin fin) {
   const int L = cta_group(G, mk), NG = (G + L - 1) / L;
-  const int group = blockIdx.x / L;
+  const int group = member / L;
   // First the group's partials (unless there is one group), then the groups'.
   double* src = partials + static_cast<int64_t>(group) * L * mk;
   int64_t stride = mk;
@@ -251,13 +253,13 @@ __device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, in
 #pragma unroll 1
   while (true) {
     __threadfence();
-    __syncthreads();
+    sync();
     if (t == 0) {
       const bool is_last = atomicAdd(arrived, 1u) == static_cast<unsigned>(count - 1);
       *s_is_last = is_last ? 1u : 0u;
       if (is_last) *arrived = 0u;  // ready for the next launch on this workspace
     }
-    __syncthreads();
+    sync();
     if (*s_is_last == 0u) return;
     __threadfence();
 #pragma unroll 1
@@ -276,6 +278,13 @@ __device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, in
     arrived = counter;
     last_level = true;
   }
+}
+
+// The same over the CTAs of a launch (partials in slot blockIdx.x).
+template <typename Skip, typename Fin>
+__device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, int mk, int t, int nthreads,
+                                         unsigned* s_is_last, Skip skip, Fin fin) {
+  sum_members(partials, counter, gridDim.x, blockIdx.x, mk, t, nthreads, s_is_last, [] { __syncthreads(); }, skip, fin);
 }
 
 // Steps 3 and 4 of the reduction: the CTA's `slots` m x k FP64 partial sums
