@@ -84,9 +84,11 @@ extern "C" tsm_status tsm_gemm_tn_f32_split(tsm_stream_t stream, int64_t n, int 
       if (e != cudaSuccess) return split_fail(e, "cudaDeviceGetAttribute");
     }
     if (!g_split_attr[dev]) {
-      e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&tsm_tn_split_tf32_kernel),
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(split::kSmemBytes));
-      if (e != cudaSuccess) return split_fail(e, "cudaFuncSetAttribute(split)");
+      for (const void* fn : {reinterpret_cast<const void*>(&tsm_tn_split_tf32_kernel<false>),
+                             reinterpret_cast<const void*>(&tsm_tn_split_tf32_kernel<true>)}) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(split::kSmemBytes));
+        if (e != cudaSuccess) return split_fail(e, "cudaFuncSetAttribute(split)");
+      }
       g_split_attr[dev] = true;
     }
   }
@@ -119,6 +121,7 @@ extern "C" tsm_status tsm_gemm_tn_f32_split(tsm_stream_t stream, int64_t n, int 
       }
     }
     SplitTmaArgs a{};
+    p.pack = 1;
     p.rows_main = n;  // the tensor maps zero-fill past row n
     p.num_chunks = (n + TmaCfg::kRows - 1) / TmaCfg::kRows;
     a.p = p;
@@ -137,11 +140,14 @@ extern "C" tsm_status tsm_gemm_tn_f32_split(tsm_stream_t stream, int64_t n, int 
     if (e != cudaSuccess) return split_fail(e, "cudaLaunchKernel(split tma)");
     return TSM_SUCCESS;
   }
+  p.pack = 32 / std::max(m, k);
   p.rows_main = rows_for_bulk(n, m, k);
   p.num_chunks = (p.rows_main + split::kRows - 1) / split::kRows;
   const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(p.num_chunks, sms));
   void* args[] = {&p};
-  e = cudaLaunchKernel(reinterpret_cast<const void*>(&tsm_tn_split_tf32_kernel), dim3(static_cast<unsigned>(grid)),
+  e = cudaLaunchKernel(p.pack > 1 ? reinterpret_cast<const void*>(&tsm_tn_split_tf32_kernel<true>)
+                                  : reinterpret_cast<const void*>(&tsm_tn_split_tf32_kernel<false>),
+                       dim3(static_cast<unsigned>(grid)),
                        dim3(split::kThreads), args, split::kSmemBytes, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return split_fail(e, "cudaLaunchKernel(split)");
   return TSM_SUCCESS;

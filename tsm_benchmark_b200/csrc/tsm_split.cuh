@@ -46,6 +46,7 @@ struct SplitArgs {
   int accumulate;
   int64_t rows_main;   // rows streamed by the pipeline; the rest (< 4) are added at the end
   int64_t num_chunks;  // ceil(rows_main / kRows)
+  int pack;            // 1-D kernel: row groups side by side in the 32 operand columns, 32 / max(m, k)
   double* partials;    // gridDim.x * m * k
   unsigned* counter;
   unsigned* error;
@@ -108,10 +109,14 @@ __device__ __forceinline__ void split_finish(const SplitArgs& p, const double (&
   double* mine = p.partials + static_cast<int64_t>(blockIdx.x) * mk;
   for (int e = t; e < mk; e += nthreads) {
     const int i = e / k, j = e - (e / k) * k;
-    // row i of C: hi part in D row i (sub-partition i / 16), lo part in row 32 + i.
-    const int hi_slot = (i >> 4) * 16 + (i & 15);
-    const int lo_slot = (2 + (i >> 4)) * 16 + (i & 15);
-    mine[e] = red[hi_slot * 32 + j] + red[lo_slot * 32 + j];
+    // row i of C: hi part in D row i, lo part in row 32 + i; packed row groups
+    // have theirs in the diagonal blocks.
+    double s = 0.0;
+    for (int g = 0; g < p.pack; ++g) {
+      const int row = g * m + i, col = g * k + j;
+      s += red[row * 32 + col] + red[(32 + row) * 32 + col];
+    }
+    mine[e] = s;
   }
   split_finish_ctas(p, t, nthreads, s_is_last);
 }
@@ -132,6 +137,12 @@ __device__ __forceinline__ void split_finish_ctas(const SplitArgs& p, int t, int
       });
 }
 
+// PACKED: p.pack > 1, narrow operands (below); otherwise one chunk per tile.
+// B200, 200 MB of operands, one chunk per tile -> packed, us: 1 x 1 2041 -> 216,
+// 3 x 3 694 -> 112, 5 x 6 390 -> 100, 10 x 10 222 -> 93, 15 x 16 152 -> 92; the
+// results differ by FP64 rounding alone (1.4e-16).  A kernel of its own: with
+// the packed addressing compiled into the other one, 16 x 17 took 178 us, not 135.
+template <bool PACKED>
 __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(const SplitArgs p) {
   using namespace split;
   extern __shared__ unsigned char smem_raw[];
@@ -181,8 +192,26 @@ __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(c
   dev::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  int64_t nchunks_mine = 0;
-  for (int64_t c = blockIdx.x; c < p.num_chunks; c += G) ++nchunks_mine;
+  // This CTA's chunks (64 rows each, blockIdx.x + i G), two to an accumulator.
+  // Narrow operands leave most of the 32 columns of a tile empty, so `pack`
+  // such pairs share one, side by side: tile 2 I + h holds chunk 2 (pack I + g)
+  // + h in columns g m .. (g k ..).  Each diagonal block of D then sees the same
+  // products in the same order as an accumulator of its own (the blocks off the
+  // diagonal are ignored), and a chunk costs 1 / pack of the tile's conversions,
+  // MMAs and drain, which are what bounds this kernel.
+  int64_t mine = 0;
+  for (int64_t c = blockIdx.x; c < p.num_chunks; c += G) ++mine;
+  const int pack = PACKED ? p.pack : 1;
+  const int64_t pairs = (mine + 1) / 2, sets = (pairs + pack - 1) / pack;
+  // the last set's second tile is empty if its only pair has one chunk
+  const int64_t nchunks_mine = !PACKED ? mine : mine == 0 ? 0 : 2 * sets - (pairs - (sets - 1) * pack == 1 && (mine & 1) ? 1 : 0);
+  // rows of slot g in tile `it` (0: no such chunk) and the first one's index
+  auto slot_rows = [&](int64_t it, int g, int64_t& r0) {
+    const int64_t i = PACKED ? 2 * (pack * (it >> 1) + g) + (it & 1) : it;
+    r0 = (blockIdx.x + i * G) * kRows;
+    const int64_t left = i < mine ? p.rows_main - r0 : 0;
+    return static_cast<int>(left < kRows ? left : kRows);
+  };
 
   double acc[32];
 #pragma unroll
@@ -192,27 +221,32 @@ __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(c
     // ---------------- TMA producer
     const uint64_t policy = dev::policy_evict_first();
     for (int64_t it = 0; it < nchunks_mine; ++it) {
-      const int64_t c = blockIdx.x + it * G;
       const int s = static_cast<int>(it % kRawStages);
       bool ok = true;
-      if (lane == 0) {
-        if (it >= kRawStages)
-          ok = dev::mbar_wait(&raw_empty[s], static_cast<uint32_t>(((it / kRawStages) - 1) & 1), abort);
-        if (ok) {
-          const int64_t r0 = c * kRows;
-          const int64_t rows = (p.rows_main - r0) < kRows ? (p.rows_main - r0) : kRows;
-          const uint32_t ba = static_cast<uint32_t>(rows * m * 4), bb = static_cast<uint32_t>(rows * k * 4);
-          unsigned char* st = raw_ring + s * kRawStageBytes;
-          dev::mbar_arrive_expect_tx(&raw_full[s], ba + bb);
-          dev::bulk_g2s_evict_first(st, p.A + r0 * m, ba, &raw_full[s], policy);
-          dev::bulk_g2s_evict_first(st + kRows * 32 * 4, p.B + r0 * k, bb, &raw_full[s], policy);
-        } else {
+      if (lane == 0 && it >= kRawStages)
+        ok = dev::mbar_wait(&raw_empty[s], static_cast<uint32_t>(((it / kRawStages) - 1) & 1), abort);
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      if (!ok) {
+        if (lane == 0) {
           *abort = 1;
           atomicOr(p.error, dev::kErrTimeout);
         }
+        break;
       }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      if (!ok) break;
+      // lane g copies slot g's rows
+      int64_t r0 = 0;
+      const int rows = lane < pack ? slot_rows(it, lane, r0) : 0;
+      const unsigned all = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(rows));
+      if (lane == 0) dev::mbar_arrive_expect_tx(&raw_full[s], all * static_cast<unsigned>((m + k) * 4));
+      __syncwarp();
+      if (rows > 0) {
+        unsigned char* st = raw_ring + s * kRawStageBytes;
+        dev::bulk_g2s_evict_first(st + lane * kRows * m * 4, p.A + r0 * m, static_cast<uint32_t>(rows * m * 4),
+                                  &raw_full[s], policy);
+        dev::bulk_g2s_evict_first(st + kRows * 32 * 4 + lane * kRows * k * 4, p.B + r0 * k,
+                                  static_cast<uint32_t>(rows * k * 4), &raw_full[s], policy);
+      }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (lane 0); the warp stays converged.
@@ -251,8 +285,20 @@ __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(c
   } else if (warp < kEpiWarp0) {
     // ---------------- converters: raw FP32 -> TF32 hi / lo operand tiles
     const int ct = t - 64;  // 0 .. 255
+    // PACKED: a thread's 4 columns (chunk ct & 7) are the same in every tile;
+    // where each lies in the raw stage (row 0), and its slot (-1: past the last).
+    int at[2][4], slot[2][4];
+    if constexpr (PACKED) {
+#pragma unroll
+      for (int which = 0; which < 2; ++which)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int w = which ? k : m, col = 4 * (ct & 7) + e, g = col / w;
+          slot[which][e] = g < pack ? g : -1;
+          at[which][e] = g < pack ? (g * kRows) * w + col - g * w : 0;
+        }
+    }
     for (int64_t it = 0; it < nchunks_mine; ++it) {
-      const int64_t c = blockIdx.x + it * G;
       const int s = static_cast<int>(it % kRawStages);
       const int o = static_cast<int>(it % kOpStages);
       bool ok = dev::mbar_wait(&raw_full[s], static_cast<uint32_t>((it / kRawStages) & 1), abort);
@@ -263,8 +309,9 @@ __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(c
         atomicOr(p.error, dev::kErrTimeout);
         break;
       }
-      const int64_t r0 = c * kRows;
-      const int rows = static_cast<int>((p.rows_main - r0) < kRows ? (p.rows_main - r0) : kRows);
+      int64_t r0;
+      const bool whole = it < 2 * (sets - 1);  // PACKED: every slot holds a whole chunk
+      const int rows = PACKED ? 0 : slot_rows(it, 0, r0);
       const float* rawA = reinterpret_cast<const float*>(raw_ring + s * kRawStageBytes);
       const float* rawB = rawA + kRows * 32;
       unsigned char* opA = op_ring + o * kOpStageBytes;
@@ -272,22 +319,28 @@ __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(c
       // 2 operands x 64 rows x 8 chunks = 1024 chunk jobs over 256 threads.
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int job = ct + q * 256;
-        const int which = job >> 9;  // 0: A, 1: B
-        const int r = (job >> 3) & 63;
-        const int ch = job & 7;
+        const int which = q >> 1;  // 0: A, 1: B
+        const int r = ((ct + q * 256) >> 3) & 63;
+        const int ch = ct & 7;
         const int w = which ? k : m;
-        const float* src = (which ? rawB : rawA) + r * w;
+        const float* raw = (which ? rawB : rawA) + r * w;
         float x[4];
-        if (w == 32 && r < rows) {
-          const float4 v = reinterpret_cast<const float4*>(src)[ch];
+        if (!PACKED && w == 32 && r < rows) {
+          const float4 v = reinterpret_cast<const float4*>(raw)[ch];
           x[0] = v.x;
           x[1] = v.y;
           x[2] = v.z;
           x[3] = v.w;
+        } else if (!PACKED) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[e] = (r < rows && 4 * ch + e < w) ? raw[4 * ch + e] : 0.0f;
+        } else if (whole) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[e] = slot[which][e] >= 0 ? raw[at[which][e]] : 0.0f;
         } else {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) x[e] = (r < rows && 4 * ch + e < w) ? src[4 * ch + e] : 0.0f;
+          for (int e = 0; e < 4; ++e)
+            x[e] = slot[which][e] >= 0 && r < slot_rows(it, slot[which][e], r0) ? raw[at[which][e]] : 0.0f;
         }
         float4 hi, lo;
         hi.x = dev::to_tf32(x[0]);
