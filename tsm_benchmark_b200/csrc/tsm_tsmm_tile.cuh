@@ -14,7 +14,8 @@
 //     there), and a storing warp writes the chunk's rows with ONE bulk copy:
 //     whole 128-byte lines whatever q is.
 // The sum over p runs in the order of tsm_tsmm_dmma.cuh (k-step 2 kb + e:
-// columns 8 kb + 2 t + e), so the two agree bit for bit.
+// columns 8 kb + 2 t + e).  Up to 7 columns on either side lanes take whole
+// rows instead (tsmm_rows).
 //
 // 16 consumer warps, four a scheduler: with 8 the chain of a unit (loads,
 // dependent MMAs, stores) left the tensor pipe idle (13 x 13 FP64, 400 MB: 110
@@ -54,6 +55,13 @@ struct TsmmTileArgs {
 // k-steps of 4 of p columns (pairs of them beyond p = 4) and 8-column tiles of q.
 __host__ __device__ constexpr int tsmm_ksteps(int p) { return p <= 4 ? 1 : 2 * ((p + 7) / 8); }
 __host__ __device__ constexpr int tsmm_tiles(int q) { return (q + 7) / 8; }
+// Rows to lanes instead of tiles: an 8 x 8 MMA tile is mostly padding there,
+// and a row's p q multiplications cost less than its bytes.  B200, 400 MB read
+// and written, backward, MMA units -> rows to lanes, us: FP64 1 x 1 210 -> 71,
+// 3 x 3 87 -> 66, 7 x 7 71 -> 65; FP32 2 x 4 156 -> 86, 3 x 3 155 -> 77, 7 x 7
+// 103 -> 92.  At 8 columns the rows' stride meets bank conflicts: 5 x 8 FP64 69
+// -> 91.
+__host__ __device__ constexpr bool tsmm_narrow(int p, int q) { return p <= 7 && q <= 7; }
 
 namespace detail {
 
@@ -176,6 +184,47 @@ __device__ __forceinline__ void tsmm_unit(const T* x, T* y, const double* wf, in
   }
 }
 
+// Narrow problems: a lane takes a row, its P values in registers and W (p x q
+// doubles, row-major) broadcast from shared memory.  A unit is 32 rows.
+template <int P, bool BETA, typename T>
+__device__ __forceinline__ int tsmm_rows(const T* x, T* y, const double* w, int q, int rows, int u, int lane) {
+  const int units = (rows + 31) / 32;
+#pragma unroll 1
+  for (; u < units; u += kTsmmTileCW) {
+    const T* xr = x + (32 * u + lane) * P;
+    T* yr = y + (32 * u + lane) * q;
+    double v[P];
+    if constexpr (P % 2 == 0) {
+#pragma unroll
+      for (int a = 0; a < P; a += 2) load_pair(xr + a, v[a], v[a + 1]);
+    } else {
+#pragma unroll
+      for (int a = 0; a < P; ++a) v[a] = static_cast<double>(xr[a]);
+    }
+#pragma unroll 4
+    for (int o = 0; o < q; ++o) {
+      double s = v[0] * w[o];
+#pragma unroll
+      for (int a = 1; a < P; ++a) s = fma(v[a], w[a * q + o], s);
+      yr[o] = static_cast<T>(BETA ? s + static_cast<double>(yr[o]) : s);
+    }
+  }
+  return u - units;
+}
+
+template <bool BETA, typename T>
+__device__ __forceinline__ int tsmm_rows(const T* x, T* y, const double* w, int p, int q, int rows, int u, int lane) {
+  switch (p) {
+    case 1: return tsmm_rows<1, BETA>(x, y, w, q, rows, u, lane);
+    case 2: return tsmm_rows<2, BETA>(x, y, w, q, rows, u, lane);
+    case 3: return tsmm_rows<3, BETA>(x, y, w, q, rows, u, lane);
+    case 4: return tsmm_rows<4, BETA>(x, y, w, q, rows, u, lane);
+    case 5: return tsmm_rows<5, BETA>(x, y, w, q, rows, u, lane);
+    case 6: return tsmm_rows<6, BETA>(x, y, w, q, rows, u, lane);
+    default: return tsmm_rows<7, BETA>(x, y, w, q, rows, u, lane);
+  }
+}
+
 // This warp's units of a chunk, from unit `u` on; returns the first one past the chunk.
 template <int RG, bool BETA, bool XP, bool YP, typename T>
 __device__ __forceinline__ int tsmm_units(const T* x, T* y, const double* wf, int p, int q, int rows, int u, int lane) {
@@ -289,6 +338,14 @@ __global__ void __launch_bounds__(kTsmmTileThreads, 1) tsm_tsmm_tile_kernel(cons
     for (int pi = 0; pi < args.a.nprob; ++pi) {
       const TsmmProblem<T>& pr = args.a.prob[pi];
       double* wf = reinterpret_cast<double*>(smem + args.w_offset[pi]);
+      if (tsmm_narrow(pr.p, pr.q)) {
+        for (int f = tid; f < pr.p * pr.q; f += CW * 32) {
+          const int a = f / pr.q, o = f - a * pr.q;
+          const double w = static_cast<double>(pr.W[a * pr.w_row + o * pr.w_col]);
+          wf[f] = pr.negate ? -w : w;
+        }
+        continue;
+      }
       const int ks = tsmm_ksteps(pr.p), nt = tsmm_tiles(pr.q);
       for (int f = warp; f < ks * nt; f += CW) {
         const int s = f / nt, j = f - s * nt;
@@ -322,6 +379,10 @@ __global__ void __launch_bounds__(kTsmmTileThreads, 1) tsm_tsmm_tile_kernel(cons
         break;
       }
       __syncwarp();
+      if (tsmm_narrow(p, q)) {
+        turn = pr.beta ? detail::tsmm_rows<true>(x, y, wf, p, q, rows, turn, lane)
+                       : detail::tsmm_rows<false>(x, y, wf, p, q, rows, turn, lane);
+      } else
       switch ((pr.beta ? 4 : 0) | (p & 1 ? 0 : 2) | (q & 1 ? 0 : 1)) {
         case 0: turn = detail::tsmm_units<false, false, false>(x, y, wf, p, q, rows, turn, lane); break;
         case 1: turn = detail::tsmm_units<false, false, true>(x, y, wf, p, q, rows, turn, lane); break;
