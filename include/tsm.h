@@ -86,7 +86,7 @@ tsm_status tsm_gemm_tn_f64_variant(tsm_stream_t stream, int64_t n, int m, int k,
 /* Same as tsm_gemm_tn_f64_variant, launching at most max_ctas CTAs (<= 0:
  * the variant's own grid, one or a few CTAs per SM; max_ctas never raises
  * it).  Every kernel deals its rows over whatever grid it gets, so the
- * result is the same product; the last CTA's sum over the per-CTA partials
+ * result is the same product; the sum over the per-CTA partials
  * follows the grid, so bits may differ from another grid's.  Replaces the
  * launch-size parameters of the reference: `stride` (the work-item count of
  * tsmttsm.hh:15-439 and of the generated kernels, sycl_codegen.py:466,
@@ -202,8 +202,8 @@ tsm_status tsm_gram_f64(tsm_stream_t stream, int64_t n, int m, const double* A, 
  * n <= 2^31 - 8193 (values of r contiguous, columns zero-padded to the
  * kernel's capacity);
  * FP64 tensor cores when the widths rounded up to powers of two multiply to
- * more than 64.  Any other layout (mixed, odd pitches, unaligned) runs a
- * register-tile kernel with strided loads: correct, not tuned.  No
+ * more than 64.  Any other layout (mixed, odd pitches, unaligned) runs on
+ * the FP64 tensor cores with each operand loaded its own way.  No
  * counterpart in the reference, whose operands are always row-major with
  * pitch M (tsmttsm.hh:15-35; sycl_codegen_new.py:66-67).  Same workspace as
  * tsm_gemm_tn_f64 (tsm_gemm_tn_workspace_size(n, m, k)). */

@@ -91,8 +91,8 @@ __device__ __forceinline__ uint32_t op_offset(int r, int c) {
 // epi0..epi0+3, lanes 0-15: D row 16 (w % 4) + lane, 32 columns) -> `red`
 // (16 KB of shared memory no longer in use), the CTA's m x k partial (D rows
 // i and 32 + i -- the hi and lo parts of A's column i -- added) into the
-// workspace, and the last CTA's fixed-order sum over CTAs (plus the rows
-// [rows_main, n) the pipeline left) into C.
+// workspace, and the fixed-order sum over CTAs (plus the rows [rows_main, n)
+// the pipeline left) into C.
 __device__ __forceinline__ void split_finish_ctas(const SplitArgs& p, int t, int nthreads, unsigned* s_is_last);
 
 __device__ __forceinline__ void split_finish(const SplitArgs& p, const double (&acc)[32], double* red, int t,

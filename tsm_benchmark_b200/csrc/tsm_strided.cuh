@@ -36,9 +36,9 @@
 // on the tile kernel (tsm_tile.cuh).
 //
 // Both end in the deterministic two-level reduction of tsm_plain.cuh
-// (finish_partials): per-CTA partials in the workspace, the last CTA sums
-// them in CTA order.  Every wait is bounded (dev::mbar_wait); a timeout sets
-// the error word, drains the CTA's copies (bounded) and returns.
+// (finish_partials): per-CTA partials in the workspace, summed in CTA order.
+// Every wait is bounded (dev::mbar_wait); a timeout sets the error word, drains
+// the CTA's copies (bounded) and returns.
 #pragma once
 
 #include <cuda.h>
