@@ -197,7 +197,9 @@ const TunedTables& tuned() {
 int tuned_variant(const std::vector<TunedEntry>& entries, int dtype, int64_t n, int m, int k, const void* A,
                   int64_t lda, const void* B, int64_t ldb, bool tiles = true) {
   for (auto e = entries.rbegin(); e != entries.rend(); ++e)
-    if (e->nmin <= n && (tiles || variants()[e->variant]->kind != kKindTile) && applicable(variants()[e->variant], dtype, n, m, k, A, lda, B, ldb)) return e->variant;
+    if (e->nmin <= n && (tiles || variants()[e->variant]->kind != kKindTile) &&
+        applicable(variants()[e->variant], dtype, n, m, k, A, lda, B, ldb))
+      return e->variant;
   return -1;
 }
 

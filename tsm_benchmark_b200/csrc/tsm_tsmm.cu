@@ -343,7 +343,8 @@ tsm_status launch_tsmm(cudaStream_t stream, TsmmProblem<T>* probs, int nprob, vo
     }
   }
   const int sms = g_sms[dev];
-  if (bulk && prefers_tile(probs, nprob)) return launch_tile<T>(stream, dev, sms, probs, nprob, reinterpret_cast<unsigned*>(ws) + 1);
+  if (bulk && prefers_tile(probs, nprob))
+    return launch_tile<T>(stream, dev, sms, probs, nprob, reinterpret_cast<unsigned*>(ws) + 1);
   if (bulk) return launch_dmma<T>(stream, dev, sms, probs, nprob, reinterpret_cast<unsigned*>(ws) + 1);
 
   int idx = -1;
