@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
                   detail::store_pair(ybase + (rb + 8 * i) * Q + 8 * j, d[i][j][0], d[i][j][1], 0);
               }
           }
+          if (Q < 8) __syncwarp();  // half the lanes stored; the next rows' MMAs take the whole warp
         }
       } else
       for (int rb = slot * K::BLK; rb < rows; rb += K::PASS) {
@@ -298,12 +299,21 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
 #pragma unroll
             for (int i = 0; i < K::RG; ++i) detail::load_pair(xr[i] + kappa, a[i][0], a[i][1]);
           } else {
+            // Columns at or past p read a valid one and are replaced by zeros with
+            // a select: no lane may branch around a load here, or the warp could
+            // reach the warp-wide MMAs in two parts, which never end.
+            const int c0 = min(kappa, p - 1), c1 = min(kappa + 1, p - 1);
 #pragma unroll
             for (int i = 0; i < K::RG; ++i) {
-              a[i][0] = kappa < p ? static_cast<double>(xr[i][kappa]) : 0.0;
-              a[i][1] = K::KPL == 2 && kappa + 1 < p ? static_cast<double>(xr[i][kappa + 1]) : 0.0;
+              const double v0 = static_cast<double>(xr[i][c0]);
+              a[i][0] = kappa < p ? v0 : 0.0;
+              if constexpr (K::KPL == 2) {
+                const double v1 = static_cast<double>(xr[i][c1]);
+                a[i][1] = kappa + 1 < p ? v1 : 0.0;
+              }
             }
           }
+          __syncwarp();
 #pragma unroll
           for (int e = 0; e < K::KPL; ++e)
 #pragma unroll
