@@ -22,3 +22,36 @@ def test_no_conditional_load_in_the_mma_kernels():
     for f in files:
         hits = [m.group(0) for m in load.finditer(_code(f))]
         assert not hits, (os.path.basename(f), hits)
+
+
+def _enclosing(code, at):
+    """Headers of the blocks around position `at`, innermost first."""
+    depth = 0
+    for i in range(at - 1, -1, -1):
+        if code[i] == "}":
+            depth += 1
+        elif code[i] == "{":
+            if depth:
+                depth -= 1
+                continue
+            start = max(code.rfind(c, 0, i) for c in "{}") + 1
+            yield code[start:i]
+
+
+def test_a_warp_gives_up_a_wait_as_one():
+    """A bounded wait of one lane (dev::mbar_wait) stands only where one lane
+    runs, or directly before a vote (dev::warp_agrees); warps wait with one
+    verdict (dev::mbar_wait_warp), or a lane that gave up would leave the others
+    at the next warp-wide instruction."""
+    single = re.compile(r"lane == 0|\bbool cm_produce\(|\bvoid cm_drain\(")
+    seen = 0
+    for f in glob.glob(os.path.join(CSRC, "*.cuh")):
+        code = _code(f)
+        for m in re.finditer(r"dev::mbar_wait\(", code):
+            seen += 1
+            statement = code[max(code.rfind(c, 0, m.start()) for c in ";{}") + 1:m.start()]
+            heads = [statement, *_enclosing(code, m.start())]
+            voted = re.search(r"^[^{}]*dev::warp_agrees\(ok\)", code[m.end():])
+            assert voted or any(single.search(h.split(";")[-1]) for h in heads), (
+                os.path.basename(f), code[m.start() - 80:m.end() + 60])
+    assert seen >= 20

@@ -185,11 +185,10 @@ __device__ __forceinline__ void consume_segment(const BatchedArgs& a, const Batc
 
   for (int64_t r0 = seg.r0; r0 < seg.r1; r0 += RS, ++it) {
     const int s = static_cast<int>(it % kStages);
-    if (!*abort && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / kStages) & 1), abort)) {
+    if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / kStages) & 1), abort)) {
       *abort = 1;
       atomicOr(a.error, dev::kErrTimeout);
-    }
-    if (!*abort) {
+    } else {
       const int rows = static_cast<int>((seg.r1 - r0) < RS ? (seg.r1 - r0) : RS);
       const double* sa = reinterpret_cast<const double*>(ring + s * kStageBytes) + colA;
       const double* sb = reinterpret_cast<const double*>(ring + s * kStageBytes) + RS * M + colB;
@@ -255,11 +254,10 @@ __device__ __forceinline__ void consume_segment_dmma(const BatchedArgs& a, const
 
   for (int64_t r0 = seg.r0; r0 < seg.r1; r0 += RS, ++it) {
     const int s = static_cast<int>(it % kStages);
-    if (!*abort && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / kStages) & 1), abort)) {
+    if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / kStages) & 1), abort)) {
       *abort = 1;
       atomicOr(a.error, dev::kErrTimeout);
-    }
-    if (!*abort) {
+    } else {
       const int rows = static_cast<int>((seg.r1 - r0) < RS ? (seg.r1 - r0) : RS);
       const unsigned char* stage = ring + s * kStageBytes;
 #pragma unroll 2

@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(BulkKernel<T, WA, WB, TA, TB, CW, STAGES, RS, 
     int64_t it = 0;
     for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      if (!dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
         *abort = 1;
         atomicOr(p.error, dev::kErrTimeout);
         break;

@@ -279,12 +279,11 @@ __global__ void __launch_bounds__(kTileThreads, 1) tsm_tn_tile_kernel(const __gr
     int64_t it = 0;
     for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      if (!dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
         *abort = 1;
         atomicOr(p.error, dev::kErrTimeout);
         break;
       }
-      __syncwarp();
       const unsigned char* stage = smem + s * args.stage_bytes;
       const T* sa = reinterpret_cast<const T*>(stage + xa.offset) + xa.first + base_a;
       const T* sb = reinterpret_cast<const T*>(stage + xb.offset) + xb.first + base_b;

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
         detail::load_w_frags<TX, K::KS, K::NT>(pr, o0, g, t, b);
         cur = pi;
       }
-      if (!dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
         *abort = 1;
         atomicOr(args.error, dev::kErrTimeout);
         break;

@@ -373,12 +373,11 @@ __global__ void __launch_bounds__(kTsmmTileThreads, 1) tsm_tsmm_tile_kernel(cons
       const T* x = reinterpret_cast<const T*>(stage);
       T* y = reinterpret_cast<T*>(const_cast<unsigned char*>(stage) + args.y_offset[pi]);
       const double* wf = reinterpret_cast<const double*>(smem + args.w_offset[pi]);
-      if (!dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
         *abort = 1;
         atomicOr(args.a.error, dev::kErrTimeout);
         break;
       }
-      __syncwarp();
       if (tsmm_narrow(p, q)) {
         turn = pr.beta ? detail::tsmm_rows<true>(x, y, wf, p, q, rows, turn, lane)
                        : detail::tsmm_rows<false>(x, y, wf, p, q, rows, turn, lane);
