@@ -193,13 +193,26 @@ const TunedTables& tuned() {
   return *tables;
 }
 
-// The entry with the largest nmin <= n whose variant takes the request, or -1.
+bool pitched_prefers_tile(bool f64, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb);
+
+// The entry with the largest nmin <= n, if it holds for the operands, or -1.  The
+// table was timed on dense, aligned operands.  Others keep its choice among the
+// tensor-box kernels, which load any 16-byte pitch as they load dense rows, and
+// a tile kernel where the rule for pitched rows agrees; the bulk kernels do not
+// take them, and an entry for fewer rows, or a kernel that was the best on
+// dense rows, says nothing about theirs (narrow slices of 8 x 4 at 3 x 10^6 rows
+// took the tile kernel that had won on 4096 dense ones: 123 us, direct 71).
 int tuned_variant(const std::vector<TunedEntry>& entries, int dtype, int64_t n, int m, int k, const void* A,
                   int64_t lda, const void* B, int64_t ldb, bool tiles = true) {
-  for (auto e = entries.rbegin(); e != entries.rend(); ++e)
-    if (e->nmin <= n && (tiles || variants()[e->variant]->kind != kKindTile) &&
-        applicable(variants()[e->variant], dtype, n, m, k, A, lda, B, ldb))
-      return e->variant;
+  const bool dense = lda == m && ldb == k && aligned16(A) && aligned16(B);
+  for (auto e = entries.rbegin(); e != entries.rend(); ++e) {
+    const Variant* v = variants()[e->variant];
+    if (e->nmin > n || (!tiles && v->kind == kKindTile)) continue;
+    if (!applicable(v, dtype, n, m, k, A, lda, B, ldb)) return -1;
+    const bool holds = dense || v->kind == kKindDmma ||
+                       (v->kind == kKindTile && pitched_prefers_tile(dtype == kF64, n, m, k, A, lda, B, ldb));
+    return holds ? e->variant : -1;
+  }
   return -1;
 }
 
@@ -246,27 +259,55 @@ int tile_variant(int dtype, int m, int k) {
 // 62 -> 84, 63 x 3 61 -> 71, 13 x 8 80 -> 69, 16 x 3 91 -> 72, 20 x 3 83 -> 82,
 // 37 x 3 92 -> 75, 24 x 24 167 -> 94, 63 x 63 252 -> 238.
 //
-// Strided or unaligned rows.  The direct kernels issue a load per element and
-// lane; tensor boxes cost by the row, so narrow slices that are loaded apart
-// stay direct: SIMT -> tile, us, 1 x 8 65 -> 112, 13 x 8 100 -> 127, 13 x 13
-// 220 -> 131, 20 x 8 142 -> 66, 40 x 1 93 -> 67.  Neighbouring slices come as
-// one: FP64 3 x 3 67 -> 71, 8 x 1 66 -> 63, 8 x 8 98 -> 63, 40 x 20 720 -> 68;
-// FP32 8 x 3 74 -> 76, 5 x 5 118 -> 82, 20 x 1 77 -> 88, 40 x 1 81 -> 74.  On a
-// thousand rows narrow ones cost the same or less direct: 3 x 5 4.8 -> 5.1,
-// FP32 5 x 8 4.8 -> 5.7; 13 x 13 7.0 -> 5.5.
+// Strided or unaligned rows: pitched_prefers_tile.
 bool prefers_tile(const Variant* v, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
   const int lo = std::min(m, k), hi = std::max(m, k);
   const bool f64 = v->dtype == kF64;
-  const size_t e = f64 ? 8 : 4;
   if (v->exact) return !f64 && v->kind == kKindBulk && lo >= 16 && n * (m + k) <= int64_t(1) << 23;
-  const bool small = m * k < 100 && n < (1 << 14);
-  if (is_gram(m, k, A, lda, B, ldb)) return m >= 5 && !small;  // one load for both operands
-  if (v->kind == kKindBulk)
+  if (v->kind == kKindBulk && !is_gram(m, k, A, lda, B, ldb))
     return f64 ? m * k >= 100 || m + k >= 18 || (m + k >= 10 && n * (m + k) >= int64_t(1) << 23)
                : lo >= 8 || (hi >= 16 && hi % 8 == 0) || (lo >= 3 && hi >= 20 && hi <= 48);
-  if (tile_joint(A, m, lda, B, k, ldb, e)) return !small && (f64 ? m + k >= 8 : (lo >= 3 && m * k >= 25) || hi >= 40);
+  return pitched_prefers_tile(f64, n, m, k, A, lda, B, ldb);
+}
+
+int padded_width(int w) {
+  int p = 1;
+  while (p < w) p *= 2;
+  return p;
+}
+
+// The same for strided or unaligned rows (and A^T A, whose rows are loaded once).
+// The direct kernels issue a load per element and lane and pad widths to powers
+// of two; tensor boxes cost by the row, so narrow slices that are loaded apart
+// stay direct: SIMT -> tile, us at 300 MB, 16-byte pitches, 8 x 8 91 -> 94, 4 x
+// 16 83 -> 86, 8 x 16 87 -> 81, 7 x 20 116 -> 73; odd pitches or unaligned bases,
+// 13 x 8 80 -> 92, 16 x 4 63 -> 78, 8 x 16 74 -> 55..67, 7 x 20 110 -> 71, 13 x 13
+// 174 -> 84, 1 x 64 75 -> 50.  Within L2 the direct kernels' loads wait on its
+// latency: at 6 MB 8 x 4 10.4 -> 8.6, 16 x 4 10.0 -> 8.3, 8 x 8 FP32 10.3 -> 8.2.  At
+// 0.5 MB launch and sum decide: 1 x 64 4.8 -> 5.4, 8 x 16 5.7 -> 6.2.
+// Neighbouring slices come as one: FP64 4 x 8 54 -> 50, 8 x 8 75 -> 50, 40 x 20
+// 720 -> 68; FP32 8 x 3 74 -> 76, 5 x 5 118 -> 82, 40 x 1 81 -> 74.  In phases (an
+// odd pitch that the columns do not fill) they take four boxes for one: 4 x 4 58
+// -> 75, 8 x 4 57 -> 93, 8 x 8 59 -> 56, FP32 4 x 8 63 -> 80; within L2 the boxes
+// keep up (60 MB 4 x 4 1.2 times slower, 20 MB as fast, 6 MB 9.9 -> 8.3).  On a
+// thousand rows narrow ones cost the same or less direct: 3 x 5 4.8 -> 5.1, FP32 5
+// x 8 4.8 -> 5.7; 13 x 13 7.0 -> 5.5.
+bool pitched_prefers_tile(bool f64, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
+  const int lo = std::min(m, k), hi = std::max(m, k);
+  const int64_t e = f64 ? 8 : 4;
+  const int simt_work = padded_width(m) * padded_width(k);  // products a row
+  const bool small = m * k < 100 && n < (1 << 14);
+  if (is_gram(m, k, A, lda, B, ldb)) return m >= 5 && !small;  // one load for both operands
+  bool phases = false;
+  if (tile_joint(A, m, lda, B, k, ldb, static_cast<size_t>(e), &phases)) {
+    if (phases && simt_work < 64 && n * (m + k) * e >= int64_t(32) << 20) return false;
+    return !small && (f64 ? m + k >= 8 : (lo >= 3 && m * k >= 25) || hi >= 40);
+  }
+  const int64_t elems = n * (m + k);
+  if (f64 && simt_work < 256 && elems < (1 << 17)) return false;
+  if (simt_work >= 32 && elems >= (1 << 18) && elems * e < (16 << 20)) return true;
   const bool maps = aligned16(A) && aligned16(B) && lda * e % 16 == 0 && ldb * e % 16 == 0;
-  return m * k >= (maps ? 64 : 160) || m + k >= 28;
+  return m * k >= (maps ? 64 : 128) || m + k >= 28;
 }
 
 int default_variant(int dtype, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb,

@@ -137,8 +137,11 @@ Joint joint_columns(const void* A, int m, int64_t lda, const void* B, int k, int
 
 }  // namespace
 
-bool tile_joint(const void* A, int m, int64_t lda, const void* B, int k, int64_t ldb, size_t esize) {
-  return joint_columns(A, m, lda, B, k, ldb, esize).width > 0;
+bool tile_joint(const void* A, int m, int64_t lda, const void* B, int k, int64_t ldb, size_t esize, bool* phases) {
+  const Joint j = joint_columns(A, m, lda, B, k, ldb, esize);
+  const bool aligned = aligned16(j.a_first == 0 ? A : B);
+  *phases = !(aligned && (lda == j.width || lda * int64_t(esize) % 16 == 0));
+  return j.width > 0;
 }
 
 template <typename T>

@@ -21,8 +21,9 @@ template <typename T>
 tsm_status launch_tile(const Variant* v, int sms, cudaStream_t stream, PlainArgs<T> p, int64_t a_row, int64_t a_col,
                        int64_t b_row, int64_t b_col, int64_t max_ctas);
 
-// Whether row-major operands would be loaded as one (neighbouring column blocks of one matrix).
-bool tile_joint(const void* A, int m, int64_t lda, const void* B, int k, int64_t ldb, size_t esize);
+// Whether row-major operands would be loaded as one (neighbouring column blocks of
+// one matrix), and whether in phases rather than by bulk copies or whole boxes.
+bool tile_joint(const void* A, int m, int64_t lda, const void* B, int k, int64_t ldb, size_t esize, bool* phases);
 
 // launch_tile for the strided entry point: picks the variant, prepares it on the
 // current device and checks the workspace.
