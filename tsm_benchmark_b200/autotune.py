@@ -54,16 +54,18 @@ def candidates(variants: list[dict], m: int, k: int, dtype: str = "f64") -> list
     """Variants of `dtype` that accept (m, k) for distinct A and B: every
     exact one, and the capacity ones no more than twice the smallest capacity
     per side (larger ones only add masked work); of the any-layout
-    tensor-core ones only the one with the least capacities.  Gram variants
-    (B is A) are not candidates."""
+    tensor-core ones, which take m x k and k x m, only the one with the least
+    capacities, listed with its widths in the order of the request.  Gram
+    variants (B is A) are not candidates."""
     out = []
     cm, ck = _cap(m), _cap(k)
     for v in variants:
         if v["dtype"] != dtype or v.get("gram"):
             continue
         if v["kind"] == "direct_dmma":
-            if (v["wa"], v["wb"]) == (-(-m // 8) * 8, -(-k // 8) * 8):
-                out.append(v)
+            wa, wb = -(-m // 8) * 8, -(-k // 8) * 8
+            if (v["wa"], v["wb"]) == (max(wa, wb), min(wa, wb)):
+                out.append(dict(v, wa=wa, wb=wb))
         elif v["exact"]:
             if m == v["wa"] and k == v["wb"]:
                 out.append(v)
