@@ -115,8 +115,16 @@ def _strides(x: torch.Tensor) -> tuple[int, int]:
 
 def _ld(x: torch.Tensor) -> int:
     """Leading dimension (elements between rows); strides of empty or
-    single-row tensors carry no layout, so those report their width."""
-    return max(int(x.stride(0)), int(x.shape[1])) if x.shape[0] > 1 else max(1, int(x.shape[1]))
+    single-row tensors carry no layout, so those report their width.  Rows
+    that overlap (``expand``, ``unfold``) have none: as n * width elements of
+    memory they would be read, or written, past their end."""
+    rows, width = x.shape
+    if rows <= 1:
+        return max(1, width)
+    ld = x.stride(0)
+    if ld < width or ld < 1:
+        raise ValueError(f"rows must not overlap: row stride {ld} of rows of {width} (use a contiguous copy)")
+    return ld
 
 
 _PLAIN = {torch.float64: ("tsm_gemm_tn_f64_variant", 0), torch.float32: ("tsm_gemm_tn_f32_variant", 1)}
@@ -161,12 +169,15 @@ def tsmttsm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor | None = None, *, 
     lib = _capi.load()
     with _guard(device):
         sh, ws = _launch_on(device, stream, _plain_bytes(lib, device, n, m, k))
-        if (n == 0 or m == 1 or a_col == 1) and (n == 0 or k == 1 or b_col == 1):
-            lda, ldb = (max(a_row, m), max(b_row, k)) if n > 1 else (max(1, m), max(1, k))
+        apart = n <= 1 or (a_row >= m and b_row >= k)  # rows that do not overlap
+        if apart and (n == 0 or m == 1 or a_col == 1) and (n == 0 or k == 1 or b_col == 1):
+            lda, ldb = (a_row, b_row) if n > 1 else (max(1, m), max(1, k))
             st = getattr(lib, fn_name)(sh, n, m, k, A.data_ptr(), lda, B.data_ptr(), ldb, C.data_ptr(), ldc,
                                        1 if accumulate else 0, ws.data_ptr(), ws.numel(), int(variant))
             if st:
                 _capi.check(st, fn_name)
+        elif not f64:  # unit column strides (checked), so A or B has rows that overlap
+            _ld(A), _ld(B)
         else:
             (ar, ac), (br, bc) = _strides(A), _strides(B)
             st = lib.tsm_gemm_tn_strided_f64(sh, n, m, k, A.data_ptr(), ar, ac, B.data_ptr(), br, bc, C.data_ptr(),
@@ -230,8 +241,9 @@ def default_variant(A: torch.Tensor, B: torch.Tensor) -> int:
     """Index of the variant tsmttsm() would run for these operands."""
     lib = _capi.load()
     dtype = _PLAIN[A.dtype][1] if A.dtype in _PLAIN else -1
-    return lib.tsm_gemm_tn_default_variant(dtype, A.shape[0], A.shape[1], B.shape[1], A.data_ptr(), _ld(A),
-                                           B.data_ptr(), _ld(B))
+    lda, ldb = (max(1, x.shape[1], x.stride(0) if x.shape[0] > 1 else 1) for x in (A, B))
+    return lib.tsm_gemm_tn_default_variant(dtype, A.shape[0], A.shape[1], B.shape[1], A.data_ptr(), lda,
+                                           B.data_ptr(), ldb)
 
 
 def workspace_status(device: torch.device | None = None, stream: torch.cuda.Stream | None = None) -> int:

@@ -13,13 +13,17 @@ import torch
 from .api import tsmttsm, tsmttsm_backward
 
 
+def _row_major(x: torch.Tensor) -> bool:
+    """Unit column stride and rows that do not overlap (``expand``, ``unfold``)."""
+    return x.stride(-1) == 1 and (x.shape[0] <= 1 or x.stride(0) >= x.shape[-1])
+
+
 class TSMTTSMFunction(torch.autograd.Function):
     """C = A^T B with hand-written forward and backward kernels."""
 
     @staticmethod
     def forward(ctx, A: torch.Tensor, B: torch.Tensor) -> torch.Tensor:
-        A = A if A.stride(-1) == 1 else A.contiguous()
-        B = B if B.stride(-1) == 1 else B.contiguous()
+        A, B = (x if _row_major(x) else x.contiguous() for x in (A, B))
         ctx.save_for_backward(A, B)
         return tsmttsm(A, B)
 
