@@ -12,9 +12,10 @@
 //     capacities 8, 16, 32, 48 or 64 otherwise;
 //   * anything else (mixed layouts, odd pitches, unaligned bases, overlapping
 //     strides): the tile kernel (tsm_tile.cuh), each operand loaded its own way.
-//     The register-tile kernel with a strided load per element and lane, which
-//     it replaced, ran 400 MB of 13 x 13, 20 x 8 and 40 x 40 operands, A
-//     row-major and B column-major, in 4474, 450 and 1484 us; now 97, 69 and 113.
+//     Direct loads, a strided one per element and lane, took 4474, 450 and 1484
+//     us for 400 MB of 13 x 13, 20 x 8 and 40 x 40 operands, A row-major and B
+//     column-major; the tile kernel 97, 69 and 113.  At most 8 columns of large
+//     operands they are the faster ones (direct_preferred).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -113,9 +114,13 @@ const Kernel kCmDmma[] = {CM_DMMA(8, 16), CM_DMMA(8, 32), CM_DMMA(8, 48), CM_DMM
                           CM_DMMA(32, 8), CM_DMMA(48, 8), CM_DMMA(64, 8), CM_DMMA_ROW(16), CM_DMMA_ROW(32),
                           CM_DMMA_ROW(48), CM_DMMA_ROW(64)};
 
+const Kernel kDirect[] = {Kernel{8, 8, 0, 256, StridedKernel<8, 8, 8, 8, 256>::SMEM_BYTES,
+                                 reinterpret_cast<const void*>(&tsm_tn_strided_kernel<8, 8, 8, 8, 256>)}};
+
 constexpr int kNumCmSimt = sizeof(kCmSimt) / sizeof(Kernel);
 constexpr int kNumCmDmma = sizeof(kCmDmma) / sizeof(Kernel);
-constexpr int kNumKernels = kNumCmSimt + kNumCmDmma;
+constexpr int kDirectIndex = kNumCmSimt + kNumCmDmma;
+constexpr int kNumKernels = kDirectIndex + 1;
 
 struct DeviceInfo {
   int sms = 0;
@@ -127,7 +132,7 @@ std::mutex g_mu;
 DeviceInfo g_dev[kMaxDevices];
 
 const Kernel* kernel_at(int idx) {
-  return idx < kNumCmSimt ? &kCmSimt[idx] : &kCmDmma[idx - kNumCmSimt];
+  return idx < kNumCmSimt ? &kCmSimt[idx] : idx < kDirectIndex ? &kCmDmma[idx - kNumCmSimt] : &kDirect[0];
 }
 
 int find_kernel(const Kernel* table, int count, int base, int wa, int wb) {
@@ -184,6 +189,34 @@ bool encode_transposed(CUtensorMap* map, const double* base, int64_t n, int w, i
                              swizzle, &last_error());
 }
 
+// An operand the tile kernel loads in phases whose boxes, 12 columns for 4 to 8,
+// are half fill: row-major with an odd pitch or an unaligned base, and not a
+// dense one of whole 16-byte rows.
+bool half_filled_phases(int64_t n, const double* X, int64_t s_row, int64_t s_col, int w) {
+  if (s_col != 1 || s_row < w || w < 4 || w > 6) return false;
+  return !aligned16(X) || (s_row % 2 != 0 && (s_row != w || n % 2 != 0));
+}
+
+// Whether operands of at most 8 columns run on the direct-load kernel (one 8 x 8
+// register tile a thread, rows along the lanes) rather than on the tile kernel.
+// Its loads are coalesced along the rows of column-major operands; gathers are
+// bound by the copies the producers issue, so widths that fill the register tile
+// favour it once launch and sum no longer count.  B200, tile -> direct, us:
+// column-major, odd pitch, 60 MB within L2: 8 x 8 24.7 -> 17.2, 7 x 7 25.2 -> 17.8;
+// from HBM, 400 MB: 8 x 8 131 -> 120, 7 x 7 130 -> 132, 5 x 5 133 -> 163, 2 x 2 172 ->
+// 345.  Two strides, 400 MB: 8 x 8 178 -> 148, 5 x 5 198 -> 177, 4 x 4 185 -> 197.  One
+// operand row-major and in half-filled phases, 400 MB, 5 x 5: as A 172 -> 127, as
+// B 128 -> 168.  At 8 MB the tile kernel is as fast or faster for all.  Narrower
+// column-major operands would gain within L2 (60 MB, 5 x 5 25.6 -> 20.8), and lose
+// as much when they come from HBM (28.3 -> 33.3).
+bool direct_preferred(int64_t n, int m, int k, const double* A, int64_t a_row, int64_t a_col, const double* B,
+                      int64_t b_row, int64_t b_col) {
+  if (m > 8 || k > 8 || n * (m + k) * int64_t(sizeof(double)) < int64_t(30) << 20) return false;
+  const bool rows = (a_col == 1 && a_row >= m) || (b_col == 1 && b_row >= k);
+  if (rows) return half_filled_phases(n, A, a_row, a_col, m);
+  return m + k >= (a_row == 1 && b_row == 1 ? 14 : 10);
+}
+
 }  // namespace
 }  // namespace tsm
 
@@ -225,6 +258,8 @@ extern "C" tsm_status tsm_gemm_tn_strided_f64(tsm_stream_t stream, int64_t n, in
     }
   }
   // 3. Any other strides.
+  const bool direct = idx < 0 && direct_preferred(n, m, k, A, a_row, a_col, B, b_row, b_col);
+  if (direct) idx = kDirectIndex;
   if (idx < 0)
     return run_tile_f64(static_cast<cudaStream_t>(stream), n, m, k, A, a_row, a_col, B, b_row, b_col, C, ldc, accumulate,
                         workspace, workspace_bytes);
@@ -255,6 +290,20 @@ extern "C" tsm_status tsm_gemm_tn_strided_f64(tsm_stream_t stream, int64_t n, in
   p.partials = reinterpret_cast<double*>(base + kWsHeader);
   const int64_t max_grid = static_cast<int64_t>(sms) * ctas;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
+
+  if (direct) {
+    StridedArgs a{};
+    a.p = p;
+    a.a_row = a_row;
+    a.a_col = a_col;
+    a.b_row = b_row;
+    a.b_col = b_col;
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((n + kern->threads - 1) / kern->threads, max_grid));
+    void* args[] = {&a};
+    e = cudaLaunchKernel(kern->fn, dim3(static_cast<unsigned>(grid)), dim3(kern->threads), args, kern->smem, cs);
+    if (e != cudaSuccess) return strided_fail(e, "cudaLaunchKernel(strided)");
+    return TSM_SUCCESS;
+  }
 
   CmArgs a{};
   p.num_chunks = (n + kern->rs - 1) / kern->rs;

@@ -32,10 +32,12 @@
 //     g + 2 t + s mod 8, all different.  A warp region is MT x NT tiles of
 //     C; each (group, s) unit costs MT + NT shared loads for 2 MT NT DMMAs.
 //
-// Any other positive strides (mixed layouts, odd pitches, unaligned bases) run
-// on the tile kernel (tsm_tile.cuh).
+//   * tsm_tn_strided_kernel<WA, WB, TA, TB, THREADS> -- any positive strides:
+//     TA x TB register tiles fed by read-only global loads, a row per thread
+//     group; at most 8 columns a side, where the tile kernel (tsm_tile.cuh), which
+//     takes all other strides, would be slower.
 //
-// Both end in the deterministic two-level reduction of tsm_plain.cuh
+// All three end in the deterministic two-level reduction of tsm_plain.cuh
 // (finish_partials): per-CTA partials in the workspace, summed in CTA order.
 // Every wait is bounded (dev::mbar_wait); a timeout sets the error word, drains
 // the CTA's copies (bounded) and returns.
@@ -50,6 +52,11 @@
 #include "tsm_plain.cuh"
 
 namespace tsm {
+
+struct StridedArgs {
+  PlainArgs<double> p;  // A, B, C, n, m, k, ldc, accumulate, workspace; rows_main = n
+  int64_t a_row, a_col, b_row, b_col;
+};
 
 struct CmArgs {
   PlainArgs<double> p;  // num_chunks = ceil(n / RS); rows_main = n
@@ -369,6 +376,51 @@ __global__ void __launch_bounds__(CmDmma<WA, WB, MT, NT, CW, STAGES, RS>::THREAD
   }
   __syncthreads();
   detail::finish_partials(p, red, K::S, t, K::THREADS, s_is_last);
+}
+
+// ------------------------------------------------------- any strides
+template <int WA, int WB, int TA, int TB, int THREADS>
+struct StridedKernel {
+  using S = TileShape<WA, WB, TA, TB>;
+  static_assert(THREADS % S::NT == 0 && THREADS % 32 == 0, "whole row groups, whole warps");
+  static constexpr int RG = THREADS / S::NT;  // rows per CTA step
+  static constexpr int SLOTS = S::NT < 32 ? THREADS / 32 : RG;
+  static constexpr size_t SMEM_BYTES = size_t(SLOTS) * WA * WB * sizeof(double) + 16;
+};
+
+template <int WA, int WB, int TA, int TB, int THREADS>
+__global__ void __launch_bounds__(THREADS) tsm_tn_strided_kernel(const StridedArgs args) {
+  using K = StridedKernel<WA, WB, TA, TB, THREADS>;
+  using S = typename K::S;
+  const PlainArgs<double>& p = args.p;
+  extern __shared__ __align__(128) unsigned char smem[];
+  unsigned* s_is_last = reinterpret_cast<unsigned*>(smem + K::SMEM_BYTES - 16);
+
+  const int t = threadIdx.x;
+  const int tile = t % S::NT;
+  const int ta = tile % S::QA, tb = tile / S::QA;
+  const int colA = ta * TA, colB = tb * TB;
+  const int validA = p.m - colA, validB = p.k - colB;
+
+  double acc[TA][TB];
+#pragma unroll
+  for (int i = 0; i < TA; ++i)
+#pragma unroll
+    for (int j = 0; j < TB; ++j) acc[i][j] = 0.0;
+
+  const int64_t rstep = static_cast<int64_t>(gridDim.x) * K::RG;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * K::RG + t / S::NT; r < p.n; r += rstep) {
+    const double* ar = p.A + r * args.a_row + colA * args.a_col;
+    const double* br = p.B + r * args.b_row + colB * args.b_col;
+    double a[TA], b[TB];
+#pragma unroll
+    for (int i = 0; i < TA; ++i) a[i] = i < validA ? __ldg(ar + i * args.a_col) : 0.0;
+#pragma unroll
+    for (int j = 0; j < TB; ++j) b[j] = j < validB ? __ldg(br + j * args.b_col) : 0.0;
+    detail::outer_fma<TA, TB>(acc, a, b);
+  }
+  detail::finish_tiles<double, 2, TA, TB, S::NT, false, WA, WB>(p, acc, t, THREADS, THREADS,
+                                                                 reinterpret_cast<double*>(smem), s_is_last);
 }
 
 }  // namespace tsm
