@@ -40,9 +40,9 @@ def _enclosing(code, at):
 
 def test_a_warp_gives_up_a_wait_as_one():
     """A bounded wait of one lane (dev::mbar_wait) stands only where one lane
-    runs, or directly before a vote (dev::warp_agrees); warps wait with one
-    verdict (dev::mbar_wait_warp), or a lane that gave up would leave the others
-    at the next warp-wide instruction."""
+    runs, or where a lane that gave up still stands in at the loop's __syncwarps;
+    else warps wait with one verdict (dev::mbar_wait_warp), or that lane would leave
+    the others at the next warp-wide instruction."""
     single = re.compile(r"lane == 0|\bbool cm_produce\(|\bvoid cm_drain\(")
     seen = 0
     for f in glob.glob(os.path.join(CSRC, "*.cuh")):
@@ -51,7 +51,8 @@ def test_a_warp_gives_up_a_wait_as_one():
             seen += 1
             statement = code[max(code.rfind(c, 0, m.start()) for c in ";{}") + 1:m.start()]
             heads = [statement, *_enclosing(code, m.start())]
-            voted = re.search(r"^[^{}]*dev::warp_agrees\(ok\)", code[m.end():])
-            assert voted or any(single.search(h.split(";")[-1]) for h in heads), (
+            stands_in = re.search(r"^[^{}]*if \(!ok\) \{[^}]*for \(; it < nchunks_mine; \+\+it\) __syncwarp\(\);\s*break;",
+                                  code[m.end():])
+            assert stands_in or any(single.search(h.split(";")[-1]) for h in heads), (
                 os.path.basename(f), code[m.start() - 80:m.end() + 60])
     assert seen >= 20

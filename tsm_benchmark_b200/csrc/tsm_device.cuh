@@ -81,14 +81,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_for(bar, parity, abort, kWaitLimitNs);
 }
 
-// One verdict for a warp whose lanes each waited: all give up if one did.  A lane
-// on its own could leave the loop of a warp-wide __syncwarp, mma or barrier that
-// the others, whose try_wait still saw the phase complete, then wait in for
-// good.  Also brings the lanes together again.
-__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
-
+// The same for a whole warp, with one verdict: every lane waits, and all give up
+// if one did.  A lane on its own could leave the loop of a warp-wide
+// __syncwarp, mma or barrier that the others, whose try_wait still saw the phase
+// complete, then wait in for good.  Also brings the lanes together again.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  return warp_agrees(mbar_wait(bar, parity, abort));
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort)) != 0;
 }
 
 // 1-D bulk copy global -> this CTA's shared memory, completing `bytes` of

@@ -304,9 +304,14 @@ __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(c
       bool ok = dev::mbar_wait(&raw_full[s], static_cast<uint32_t>((it / kRawStages) & 1), abort);
       if (ok && it >= kOpStages)
         ok = dev::mbar_wait(&op_empty[o], static_cast<uint32_t>(((it / kOpStages) - 1) & 1), abort);
-      // A chunk that did not come is converted all the same, and not handed on: the
-      // vote's latency is then hidden (looked at here, it cost 32 x 32 1 %).
-      const bool go = dev::warp_agrees(ok);
+      if (!ok) {
+        *abort = 1;
+        atomicOr(p.error, dev::kErrTimeout);
+        // The lanes that go on meet at one __syncwarp a chunk: this one stands in
+        // at all that are left.  (A vote of the warp on each wait cost 2 %.)
+        for (; it < nchunks_mine; ++it) __syncwarp();
+        break;
+      }
       int64_t r0;
       const bool whole = it < 2 * (sets - 1);  // PACKED: every slot holds a whole chunk
       const int rows = PACKED ? 0 : slot_rows(it, 0, r0);
@@ -352,11 +357,6 @@ __global__ void __launch_bounds__(split::kThreads, 1) tsm_tn_split_tf32_kernel(c
         unsigned char* dst = (which ? opB : opA) + split::op_offset(r, ch);
         *reinterpret_cast<float4*>(dst) = hi;
         *reinterpret_cast<float4*>(dst + kOpHalfBytes) = lo;
-      }
-      if (!go) {
-        *abort = 1;
-        atomicOr(p.error, dev::kErrTimeout);
-        break;
       }
       dev::fence_proxy_async_smem();  // make the operand stores visible to the tensor core
       __syncwarp();

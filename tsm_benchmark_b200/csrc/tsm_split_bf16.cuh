@@ -239,9 +239,14 @@ __global__ void __launch_bounds__(split16::kThreads, 1)
       bool ok = dev::mbar_wait(&raw_full[s], static_cast<uint32_t>((it / S::RAW_STAGES) & 1), abort);
       if (ok && it >= kOpStages)
         ok = dev::mbar_wait(&op_empty[o], static_cast<uint32_t>(((it / kOpStages) - 1) & 1), abort);
-      // A chunk that did not come is converted all the same, and not handed on: the
-      // vote's latency is then hidden (looked at here, it cost 32 x 32 1 %).
-      const bool go = dev::warp_agrees(ok);
+      if (!ok) {
+        *abort = 1;
+        atomicOr(p.error, dev::kErrTimeout);
+        // The lanes that go on meet at one __syncwarp a chunk: this one stands in
+        // at all that are left.  (A vote of the warp on each wait cost 2 %.)
+        for (; it < nchunks_mine; ++it) __syncwarp();
+        break;
+      }
       const float* raw = reinterpret_cast<const float*>(smem + S::RAW_OFFSET + s * kRawStageBytes);
       unsigned char* op = smem + S::OP_OFFSET + o * S::OP_STAGE;
 #pragma unroll
@@ -265,11 +270,6 @@ __global__ void __launch_bounds__(split16::kThreads, 1)
           }
           *reinterpret_cast<uint4*>(dst + (32 * part + lane) * 128 + chunk) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-      }
-      if (!go) {
-        *abort = 1;
-        atomicOr(p.error, dev::kErrTimeout);
-        break;
       }
       dev::fence_proxy_async_smem();  // make the operand tiles visible to the tensor core
       __syncwarp();

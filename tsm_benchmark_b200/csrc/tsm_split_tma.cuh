@@ -245,9 +245,14 @@ __global__ void __launch_bounds__(split2::Cfg<ROWS, ISSUERS>::kThreads, 1)
       bool ok = dev::mbar_wait(&full[s], static_cast<uint32_t>((it / kHiStages) & 1), abort);
       if (ok && it >= kLoStages)
         ok = dev::mbar_wait(&lo_empty[o], static_cast<uint32_t>(((it / kLoStages) - 1) & 1), abort);
-      // A chunk that did not come is converted all the same, and not handed on: the
-      // vote's latency is then hidden (looked at here, it cost 32 x 32 1 %).
-      const bool go = dev::warp_agrees(ok);
+      if (!ok) {
+        *abort = 1;
+        atomicOr(p.error, dev::kErrTimeout);
+        // The lanes that go on meet at one __syncwarp a chunk: this one stands in
+        // at all that are left.  (A vote of the warp on each wait cost 2 %.)
+        for (; it < nchunks_mine; ++it) __syncwarp();
+        break;
+      }
       const uint4* hi = reinterpret_cast<const uint4*>(smem + s * kStageBytes);
       uint4* lo = reinterpret_cast<uint4*>(smem + kLoRing + o * kStageBytes);
       // A_hi and B_hi: 2 x 16 KB = 2048 16-byte vectors over 256 threads.
@@ -260,11 +265,6 @@ __global__ void __launch_bounds__(split2::Cfg<ROWS, ISSUERS>::kThreads, 1)
         w.z = lo_part(v.z);
         w.w = lo_part(v.w);
         lo[ct + q * 32 * kConvWarps] = w;
-      }
-      if (!go) {
-        *abort = 1;
-        atomicOr(p.error, dev::kErrTimeout);
-        break;
       }
       dev::fence_proxy_async_smem();  // make the lo tiles visible to the tensor core
       __syncwarp();
