@@ -236,6 +236,13 @@ int tile_variant(int dtype, int m, int k) {
   return index[(dtype * 8 + (std::max(m, k) - 1) / 8) * 8 + (std::min(m, k) - 1) / 8];
 }
 
+// The SIMT kernels are compiled for powers of two: the columns one works on for w.
+int padded_width(int w) {
+  int p = 1;
+  while (p < w) p *= 2;
+  return p;
+}
+
 // Whether an m x k product that has no tuned entry runs on the tile kernel
 // rather than on `v`, the first variant in the table that takes it.
 //
@@ -255,9 +262,14 @@ int tile_variant(int dtype, int m, int k) {
 // 24 x 24 179 -> 64, 37 x 37 463 -> 85, 63 x 63 352 -> 139 (FP64-bound).
 // Below 64 MB launch and cross-CTA sum decide: 3 x 7 at n = 200001 9.4 -> 10.7,
 // 5 x 8 at 1000 5.2 -> 5.8, 13 x 13 at 1000 7.7 -> 5.4, 64 x 5 8.6 -> 6.0.
-// FP32 (the tile kernel widens to FP64, so FP64 rate bounds it): 13 x 3
-// 62 -> 84, 63 x 3 61 -> 71, 13 x 8 80 -> 69, 16 x 3 91 -> 72, 20 x 3 83 -> 82,
-// 37 x 3 92 -> 75, 24 x 24 167 -> 94, 63 x 63 252 -> 238.
+// FP32, 300 MB.  The tile kernel widens to FP64, and the FP64 pipe bounds it on
+// narrow rows: 4 x 4 50 -> 77, 12 x 4 52 -> 62, 63 x 3 51 -> 56.  The SIMT kernels fall
+// behind where a thread holds 8 columns of either side (from 5 on: 5 x 5 79 -> 69, 6
+// x 20 87 -> 60, 13 x 8 61 -> 54), where rows of a multiple of 32 bytes put their
+// lanes on the same banks (16 x 3 70 -> 57, 40 x 2 78 -> 56, but 17 x 3 70 -> 72), and
+// where a quarter of a side padded to 64 is padding (36 x 3 74 -> 58, 48 x 3 the
+// last).  Padded to 32 the two are within 15 % (17 x 3 70 -> 72, 31 x 3 51 -> 57) and the
+// FP64 sums decide: 25 x 3 at 2^22 rows is 9e-9 off in one, 1.3e-7 in FP32.
 //
 // Strided or unaligned rows: pitched_prefers_tile.
 bool prefers_tile(const Variant* v, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
@@ -266,14 +278,8 @@ bool prefers_tile(const Variant* v, int64_t n, int m, int k, const void* A, int6
   if (v->exact) return !f64 && v->kind == kKindBulk && lo >= 16 && n * (m + k) <= int64_t(1) << 23;
   if (v->kind == kKindBulk && !is_gram(m, k, A, lda, B, ldb))
     return f64 ? m * k >= 100 || m + k >= 18 || (m + k >= 10 && n * (m + k) >= int64_t(1) << 23)
-               : lo >= 8 || (hi >= 16 && hi % 8 == 0) || (lo >= 3 && hi >= 20 && hi <= 48);
+               : lo >= 5 || (hi >= 16 && hi % 8 == 0) || (lo >= 3 && hi > 16 && hi <= 48);
   return pitched_prefers_tile(f64, n, m, k, A, lda, B, ldb);
-}
-
-int padded_width(int w) {
-  int p = 1;
-  while (p < w) p *= 2;
-  return p;
 }
 
 // The same for strided or unaligned rows (and A^T A, whose rows are loaded once).
@@ -288,8 +294,9 @@ int padded_width(int w) {
 // Neighbouring slices come as one: FP64 4 x 8 54 -> 50, 8 x 8 75 -> 50, 40 x 20
 // 720 -> 68; FP32 8 x 3 74 -> 76, 5 x 5 118 -> 82, 40 x 1 81 -> 74.  In phases (an
 // odd pitch that the columns do not fill) they take four boxes for one: 4 x 4 58
-// -> 75, 8 x 4 57 -> 93, 8 x 8 59 -> 56, FP32 4 x 8 63 -> 80; within L2 the boxes
-// keep up (60 MB 4 x 4 1.2 times slower, 20 MB as fast, 6 MB 9.9 -> 8.3).  On a
+// -> 75, 8 x 4 57 -> 93, 8 x 8 59 -> 56; within L2 the boxes keep up (60 MB 4 x 4
+// 1.2 times slower, 20 MB as fast, 6 MB 9.9 -> 8.3).  FP32 4 x 8 63 -> 80 stays, with
+// its sums in FP64.  On a
 // thousand rows narrow ones cost the same or less direct: 3 x 5 4.8 -> 5.1, FP32 5
 // x 8 4.8 -> 5.7; 13 x 13 7.0 -> 5.5.
 bool pitched_prefers_tile(bool f64, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
@@ -300,7 +307,7 @@ bool pitched_prefers_tile(bool f64, int64_t n, int m, int k, const void* A, int6
   if (is_gram(m, k, A, lda, B, ldb)) return m >= 5 && !small;  // one load for both operands
   bool phases = false;
   if (tile_joint(A, m, lda, B, k, ldb, static_cast<size_t>(e), &phases)) {
-    if (phases && simt_work < 64 && n * (m + k) * e >= int64_t(32) << 20) return false;
+    if (f64 && phases && simt_work < 64 && n * (m + k) * e >= int64_t(32) << 20) return false;
     return !small && (f64 ? m + k >= 8 : (lo >= 3 && m * k >= 25) || hi >= 40);
   }
   const int64_t elems = n * (m + k);
