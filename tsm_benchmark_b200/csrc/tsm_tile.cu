@@ -151,9 +151,9 @@ tsm_status launch_tile(const Variant* v, int sms, cudaStream_t stream, PlainArgs
   a.swap = (p.m <= v->wa && p.k <= v->wb) ? 0 : 1;
   if (p.m == 1) a_col = 1;  // a stride along an extent of one is never used
   if (p.k == 1) b_col = 1;
-  if (p.n <= 1) {
-    a_row = std::max<int64_t>(a_row, p.m * a_col);
-    b_row = std::max<int64_t>(b_row, p.k * b_col);
+  if (p.n <= 1) {  // nor a row stride, which may be more than a tensor map holds
+    a_row = p.m * a_col;
+    b_row = p.k * b_col;
   }
   p.symmetric = p.A == p.B && p.m == p.k && a_row == b_row && a_col == b_col;
   const bool row_major = a_col == 1 && b_col == 1;
