@@ -51,7 +51,7 @@ def test_a_warp_gives_up_a_wait_as_one():
             seen += 1
             statement = code[max(code.rfind(c, 0, m.start()) for c in ";{}") + 1:m.start()]
             heads = [statement, *_enclosing(code, m.start())]
-            stands_in = re.search(r"^[^{}]*if \(!ok\) \{[^}]*for \(; it < nchunks_mine; \+\+it\) __syncwarp\(\);\s*break;",
+            stands_in = re.search(r"^[^{}]*\{[^}]*for \(; (?:it|c) < [^)]*\) __syncwarp\(\);\s*break;",
                                   code[m.end():])
             assert stands_in or any(single.search(h.split(";")[-1]) for h in heads), (
                 os.path.basename(f), code[m.start() - 80:m.end() + 60])

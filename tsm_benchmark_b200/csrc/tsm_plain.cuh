@@ -478,9 +478,12 @@ __global__ void __launch_bounds__(BulkKernel<T, WA, WB, TA, TB, CW, STAGES, RS, 
     int64_t it = 0;
     for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (!dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
         *abort = 1;
         atomicOr(p.error, dev::kErrTimeout);
+        // The lanes that go on meet at one __syncwarp a chunk: this one stands in
+        // at all that are left.  (A vote of the warp on each wait cost 3 % of 8 x 8.)
+        for (; c < p.num_chunks; c += G) __syncwarp();
         break;
       }
       const int64_t r0 = c * RS;

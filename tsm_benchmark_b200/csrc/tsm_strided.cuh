@@ -173,9 +173,11 @@ __global__ void __launch_bounds__(CmSimt<WA, WB, RS, STAGES>::THREADS, 1)
     int64_t it = 0;
     for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (!dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
         *abort = 1;
         atomicOr(p.error, dev::kErrTimeout);
+        // Stands in at the remaining chunks' __syncwarps, as in tsm_plain.cuh.
+        for (; c < p.num_chunks; c += G) __syncwarp();
         break;
       }
       const double* sa = reinterpret_cast<const double*>(smem + s * K::STAGE_BYTES);
