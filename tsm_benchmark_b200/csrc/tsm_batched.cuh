@@ -148,7 +148,7 @@ __device__ __forceinline__ void finish_segment(const BatchedArgs& a, const Batch
   double* part = a.partials + seg.partial_off;
   for (int e = t; e < M * K; e += kCT) part[e] = slots(e);
   const int first = static_cast<int>(pr.seg_first);
-  detail::sum_members(
+  detail::sum_members<(M * K >= 1024)>(
       a.partials + a.segments[first].partial_off, a.counters + kCountersPerProblem * seg.problem, pr.nseg,
       si - first, M * K, t, kCT, s_flag, [] { consumer_barrier(); }, [](int) { return false; }, write);
 }

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(DmmaTn<WA, WB, MT, NT, CW, STAGES, RS>::THREAD
     }
   }
   __syncthreads();
-  detail::finish_partials(p, red, K::S, t, K::THREADS, s_is_last);
+  detail::finish_partials<WA * WB>(p, red, K::S, t, K::THREADS, s_is_last);
 }
 
 }  // namespace tsm
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(GramDmma<W, CW, STAGES, RS>::THREADS, 1)
       detail::gram_store<W, (K::R > 1 ? 1 : 0)>(sheet, lane, out);
   }
   __syncthreads();
-  detail::finish_partials(p, red, K::S, t, K::THREADS, s_is_last);
+  detail::finish_partials<W * W>(p, red, K::S, t, K::THREADS, s_is_last);
 }
 
 }  // namespace tsm

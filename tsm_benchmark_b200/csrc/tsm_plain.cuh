@@ -139,7 +139,7 @@ __device__ __forceinline__ void unrotate_tile(ACC (&acc)[TA][TB], int rotA, int 
   }
 }
 
-template <typename T>
+template <int MK, typename T>
 __device__ __forceinline__ void finish_partials(const PlainArgs<T>& p, const double* red, int slots, int t,
                                                 int nthreads, unsigned* s_is_last);
 
@@ -190,22 +190,30 @@ __device__ __forceinline__ void finish_tiles(const PlainArgs<T>& p, ACC (&acc_in
     }
   }
   __syncthreads();
-  finish_partials(p, red, slots, t, nthreads, s_is_last);
+  finish_partials<WA * WB>(p, red, slots, t, nthreads, s_is_last);
 }
 
-// The sum, in order, of `count` doubles `stride` apart, sixteen loads in
-// flight; those past `count` add -0.0, which changes no sum.
-__device__ __forceinline__ double ordered_sum(const double* src, int64_t stride, int count) {
-  double s = -0.0;
+// The sums, in order, of `count` doubles `stride` apart from src + q * step, q < E,
+// as far as q * step < left; E * W loads in flight.  Those past `count` add -0.0,
+// which changes no sum.
+template <int E, int W>
+__device__ __forceinline__ void ordered_sums(const double* src, int64_t stride, int count, int step, int left,
+                                             double (&s)[E]) {
+#pragma unroll
+  for (int q = 0; q < E; ++q) s[q] = -0.0;
 #pragma unroll 1
-  for (int b = 0; b < count; b += 16, src += 16 * stride) {
-    double v[16];
+  for (int b = 0; b < count; b += W, src += W * stride) {
+    double v[E][W];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = b + q < count ? dev::ld_cg(src + q * stride) : -0.0;
+    for (int q = 0; q < E; ++q)
 #pragma unroll
-    for (int q = 0; q < 16; ++q) s += v[q];
+      for (int w = 0; w < W; ++w)
+        v[q][w] = b + w < count && q * step < left ? dev::ld_cg(src + w * stride + q * step) : -0.0;
+#pragma unroll
+    for (int q = 0; q < E; ++q)
+#pragma unroll
+      for (int w = 0; w < W; ++w) s[q] += v[q][w];
   }
-  return s;
 }
 
 // CTAs per group of the cross-CTA sum: one group up to 32 CTAs (64 where C is
@@ -229,13 +237,19 @@ __device__ __forceinline__ int cta_group(int G, int mk) {
 // Why two levels: one CTA reading all G partials is a serial tail on one SM,
 // bound by load latency (four loads in flight a thread) and, for wide C, by
 // one SM's share of L2 bandwidth: at 64 x 64 4.8 MB from 148 CTAs.  The group
-// sums run on up to 12 SMs at once with 16 loads in flight.  On few CTAs the
-// second level's fence, atomic and load cost more than they save (4 x 4 Gram
-// at n = 10^5, 49 CTAs: 8.5 us with two levels, 7.1 with one).  B200, one
-// CTA summing -> two levels, us per call: 64 x 64 at n = 2^15 64.1 -> 32.9, at
-// 2^18 120 -> 88, at 2^21 562 -> 537; 32 x 32 at 2^15 24.4 -> 15.4; 8 x 8 at
-// 2^20 28.8 -> 26.4; 4 x 4 at 2^15 9.2 -> 7.4.
-template <typename Sync, typename Skip, typename Fin>
+// sums run on up to 12 SMs at once.  On few CTAs the second level's fence,
+// atomic and load cost more than they save (4 x 4 Gram at n = 10^5, 49 CTAs: 8.5
+// us with two levels, 7.1 with one).  B200, one CTA summing -> two levels, us
+// per call: 64 x 64 at n = 2^15 64.1 -> 32.9, at 2^18 120 -> 88, at 2^21 562 -> 537; 32
+// x 32 at 2^15 24.4 -> 15.4; 8 x 8 at 2^20 28.8 -> 26.4; 4 x 4 at 2^15 9.2 -> 7.4.
+//
+// WIDE: C has several entries a thread, summed one after another with sixteen
+// loads in flight, or, on few CTAs, where most of the sixteen would be past the
+// last, four at once with four each: whichever takes fewer rounds of L2
+// latency.  64 x 64 on 1 CTA 15.2 -> 11.8 us, on 4 15.4 -> 12.2, on 21 22.9 -> 19.4; Gram
+// 48 on 21 17.7 -> 16.1.  Narrow kernels do without: its code would lengthen
+// their few microseconds by 2 to 4 %.
+template <bool WIDE, typename Sync, typename Skip, typename Fin>
 __device__ __forceinline__ void sum_members(double* partials, unsigned* counter, int G, int member, int mk, int t,
                                             int nthreads, unsigned* s_is_last, Sync sync, Skip skip, Fin fin) {
   const int L = cta_group(G, mk), NG = (G + L - 1) / L;
@@ -262,14 +276,33 @@ __device__ __forceinline__ void sum_members(double* partials, unsigned* counter,
     sync();
     if (*s_is_last == 0u) return;
     __threadfence();
-#pragma unroll 1
-    for (int e = t; e < mk; e += nthreads) {
-      if (skip(e)) continue;
-      const double s = ordered_sum(src + e, stride, count);
+    auto put = [&](int e, double sum) {
       if (last_level)
-        fin(e, s);
+        fin(e, sum);
       else
-        src[e] = s;
+        src[e] = sum;
+    };
+    bool singly = true;
+    if constexpr (WIDE)
+      singly = (count + 15) / 16 * ((mk + nthreads - 1) / nthreads) <=
+               (count + 3) / 4 * ((mk + 4 * nthreads - 1) / (4 * nthreads));
+    if (singly) {
+#pragma unroll 1
+      for (int e = t; e < mk; e += nthreads) {
+        if (skip(e)) continue;
+        double s[1];
+        ordered_sums<1, 16>(src + e, stride, count, 0, 1, s);
+        put(e, s[0]);
+      }
+    } else if constexpr (WIDE) {
+#pragma unroll 1
+      for (int e = t; e < mk; e += 4 * nthreads) {
+        double s[4];
+        ordered_sums<4, 4>(src + e, stride, count, nthreads, mk - e, s);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (e + q * nthreads < mk && !skip(e + q * nthreads)) put(e + q * nthreads, s[q]);
+      }
     }
     if (last_level) return;
     src = partials;
@@ -281,18 +314,20 @@ __device__ __forceinline__ void sum_members(double* partials, unsigned* counter,
 }
 
 // The same over the CTAs of a launch (partials in slot blockIdx.x).
-template <typename Skip, typename Fin>
+template <bool WIDE, typename Skip, typename Fin>
 __device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, int mk, int t, int nthreads,
                                          unsigned* s_is_last, Skip skip, Fin fin) {
-  sum_members(partials, counter, gridDim.x, blockIdx.x, mk, t, nthreads, s_is_last, [] { __syncthreads(); }, skip, fin);
+  sum_members<WIDE>(partials, counter, gridDim.x, blockIdx.x, mk, t, nthreads, s_is_last, [] { __syncthreads(); }, skip,
+                    fin);
 }
 
 // Steps 3 and 4 of the reduction: the CTA's `slots` m x k FP64 partial sums
 // in `red` (shared memory, complete: the caller synchronised) are summed in
 // slot order into this CTA's workspace slot; then the CTAs' partials are
 // summed (sum_ctas), the rows [rows_main, n) the main loop left are added and
-// C is written.  Called by all `nthreads` threads of the CTA.
-template <typename T>
+// C is written.  Called by all `nthreads` threads of the CTA.  MK: the most
+// entries C has in this kernel.
+template <int MK, typename T>
 __device__ __forceinline__ void finish_partials(const PlainArgs<T>& p, const double* red, int slots, int t,
                                                 int nthreads, unsigned* s_is_last) {
   const int m = p.m, k = p.k;
@@ -306,7 +341,7 @@ __device__ __forceinline__ void finish_partials(const PlainArgs<T>& p, const dou
   }
   // 4. Symmetric (Gram): the upper triangle is summed and written to both
   //    (i, j) and (j, i), so C is exactly symmetric.
-  sum_ctas(
+  sum_ctas<(MK >= 1024)>(
       p.partials, p.counter, mk, t, nthreads, s_is_last,
       [&](int e) {
         if (!p.symmetric) return false;

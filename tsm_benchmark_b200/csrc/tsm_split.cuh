@@ -126,7 +126,7 @@ __device__ __forceinline__ void split_finish(const SplitArgs& p, const double (&
 // left, into C.
 __device__ __forceinline__ void split_finish_ctas(const SplitArgs& p, int t, int nthreads, unsigned* s_is_last) {
   const int m = p.m, k = p.k;
-  detail::sum_ctas(
+  detail::sum_ctas<false>(
       p.partials, p.counter, m * k, t, nthreads, s_is_last, [](int) { return false; },
       [&](int e, double s) {
         const int i = e / k, j = e - i * k;

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(CmSimt<WA, WB, RS, STAGES>::THREADS, 1)
       }
   }
   __syncthreads();
-  detail::finish_partials(p, red, K::CW, t, K::THREADS, s_is_last);
+  detail::finish_partials<WA * WB>(p, red, K::CW, t, K::THREADS, s_is_last);
 }
 
 // ------------------------------------------------------------------ DMMA
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(CmDmma<WA, WB, MT, NT, CW, STAGES, RS>::THREAD
     }
   }
   __syncthreads();
-  detail::finish_partials(p, red, K::S, t, K::THREADS, s_is_last);
+  detail::finish_partials<WA * WB>(p, red, K::S, t, K::THREADS, s_is_last);
 }
 
 // ------------------------------------------------------- any strides

@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tsm_tn_tile_kernel(const __gr
     }
   }
   __syncthreads();
-  detail::finish_partials(p, red, K::S, t, kTileThreads, s_is_last);
+  detail::finish_partials<64 * TA * TB>(p, red, K::S, t, kTileThreads, s_is_last);
 }
 
 }  // namespace tsm
