@@ -40,8 +40,8 @@ def _enclosing(code, at):
 
 def test_a_warp_gives_up_a_wait_as_one():
     """A bounded wait of one lane (dev::mbar_wait) stands only where one lane
-    runs, or where a lane that gave up still stands in at the loop's __syncwarps;
-    else warps wait with one verdict (dev::mbar_wait_warp), or that lane would leave
+    runs, or where a lane that gave up stays in the loop, or stands in at its
+    __syncwarps; else warps wait with one verdict (dev::mbar_wait_warp), or that lane would leave
     the others at the next warp-wide instruction."""
     single = re.compile(r"lane == 0|\bbool cm_produce\(|\bvoid cm_drain\(")
     seen = 0
@@ -53,6 +53,8 @@ def test_a_warp_gives_up_a_wait_as_one():
             heads = [statement, *_enclosing(code, m.start())]
             stands_in = re.search(r"^[^{}]*\{[^}]*for \(; (?:it|c) < [^)]*\) __syncwarp\(\);\s*break;",
                                   code[m.end():])
-            assert stands_in or any(single.search(h.split(";")[-1]) for h in heads), (
+            stays = re.search(r"if \(ok && !$", code[:m.start()]) and re.match(
+                r"[^{}]*\{\s*ok = false;\s*\*abort = 1;\s*atomicOr\([^;]*;\s*\}", code[m.end():])
+            assert stands_in or stays or any(single.search(h.split(";")[-1]) for h in heads), (
                 os.path.basename(f), code[m.start() - 80:m.end() + 60])
     assert seen >= 20

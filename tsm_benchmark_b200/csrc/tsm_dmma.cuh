@@ -163,12 +163,13 @@ __global__ void __launch_bounds__(DmmaTn<WA, WB, MT, NT, CW, STAGES, RS>::THREAD
     const int g = lane >> 2, tq = lane & 3;
     const int a_blk0 = ra * (MT / 2), b_blk0 = K::MBA + rb * (NT / 2);
     int64_t it = 0;
+    bool ok = true;  // false: a wait ran out, the remaining chunks are gone through without any
     for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (ok && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+        ok = false;  // no lane leaves the loop: its MMAs and barriers take the whole warp
         *abort = 1;
         atomicOr(p.error, dev::kErrTimeout);
-        break;
       }
       const unsigned char* stage = smem + s * K::STAGE_BYTES;
 #pragma unroll 2
@@ -314,12 +315,13 @@ __device__ __forceinline__ void gram_consume(const PlainArgs<double>& p, unsigne
 #pragma unroll
       for (int b = 0; b < 2; ++b) out[q][a][b][0] = out[q][a][b][1] = 0.0;
   int64_t it = 0;
+  bool ok = true;  // false: a wait ran out, the remaining chunks are gone through without any
   for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
     const int s = static_cast<int>(it % STAGES);
-    if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+    if (ok && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      ok = false;  // no lane leaves the loop: its MMAs and barriers take the whole warp
       *abort = 1;
       atomicOr(p.error, dev::kErrTimeout);
-      break;
     }
     const unsigned char* stage = smem + s * K::STAGE_BYTES;
 #pragma unroll 2
@@ -469,7 +471,7 @@ __global__ void __launch_bounds__(GramDmma<W, CW, STAGES, RS>::THREADS, 1)
       detail::gram_store<W, (K::R > 1 ? 1 : 0)>(sheet, lane, out);
   }
   __syncthreads();
-  detail::finish_partials<W * W>(p, red, K::S, t, K::THREADS, s_is_last);
+  detail::finish_partials<0>(p, red, K::S, t, K::THREADS, s_is_last);
 }
 
 }  // namespace tsm

@@ -246,9 +246,10 @@ __device__ __forceinline__ int cta_group(int G, int mk) {
 // WIDE: C has several entries a thread, summed one after another with sixteen
 // loads in flight, or, on few CTAs, where most of the sixteen would be past the
 // last, four at once with four each: whichever takes fewer rounds of L2
-// latency.  64 x 64 on 1 CTA 15.2 -> 11.8 us, on 4 15.4 -> 12.2, on 21 22.9 -> 19.4; Gram
-// 48 on 21 17.7 -> 16.1.  Narrow kernels do without: its code would lengthen
-// their few microseconds by 2 to 4 %.
+// latency.  64 x 64 on 1 CTA 15.2 -> 11.8 us, on 4 15.4 -> 12.2, on 21 22.9 -> 19.4.
+// Narrow kernels do without: its code would lengthen their few microseconds by
+// 2 to 4 %; so do the Gram kernels (MK = 0), which became slower by 5 us on a full
+// grid with it (64 columns, 300 MB: 103 -> 108).
 template <bool WIDE, typename Sync, typename Skip, typename Fin>
 __device__ __forceinline__ void sum_members(double* partials, unsigned* counter, int G, int member, int mk, int t,
                                             int nthreads, unsigned* s_is_last, Sync sync, Skip skip, Fin fin) {
@@ -326,7 +327,7 @@ __device__ __forceinline__ void sum_ctas(double* partials, unsigned* counter, in
 // slot order into this CTA's workspace slot; then the CTAs' partials are
 // summed (sum_ctas), the rows [rows_main, n) the main loop left are added and
 // C is written.  Called by all `nthreads` threads of the CTA.  MK: the most
-// entries C has in this kernel.
+// entries C has in this kernel, or 0 (see WIDE above).
 template <int MK, typename T>
 __device__ __forceinline__ void finish_partials(const PlainArgs<T>& p, const double* red, int slots, int t,
                                                 int nthreads, unsigned* s_is_last) {

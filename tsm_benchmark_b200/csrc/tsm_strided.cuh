@@ -322,12 +322,13 @@ __global__ void __launch_bounds__(CmDmma<WA, WB, MT, NT, CW, STAGES, RS>::THREAD
     const int g = lane >> 2, tq = lane & 3;
     const int a_row0 = 8 * ra * MT + g, b_row0 = 8 * rb * NT + g;
     int64_t it = 0;
+    bool ok = true;  // false: a wait ran out, the remaining chunks are gone through without any
     for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (ok && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+        ok = false;  // no lane leaves the loop: its MMAs and barriers take the whole warp
         *abort = 1;
         atomicOr(p.error, dev::kErrTimeout);
-        break;
       }
       const unsigned char* sa = smem + s * K::STAGE_BYTES;
       const unsigned char* sb = sa + K::TILE_A;

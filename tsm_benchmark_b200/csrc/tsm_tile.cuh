@@ -277,12 +277,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) tsm_tn_tile_kernel(const __gr
     const int base_a = 8 * K::MT * ra + g + tq * xa.t_step, base_b = 8 * K::NT * rb + g + tq * xb.t_step;
     const int ksteps = rs / 4;
     int64_t it = 0;
+    bool ok = true;  // false: a wait ran out, the remaining chunks are gone through without any
     for (int64_t c = blockIdx.x; c < p.num_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
-      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (ok && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+        ok = false;  // no lane leaves the loop: its MMAs and barriers take the whole warp
         *abort = 1;
         atomicOr(p.error, dev::kErrTimeout);
-        break;
       }
       const unsigned char* stage = smem + s * args.stage_bytes;
       const T* sa = reinterpret_cast<const T*>(stage + xa.offset) + xa.first + base_a;

@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
     int cur = -1;
     double b[K::KS][K::NT];
     int64_t it = 0;
+    bool ok = true;  // false: a wait ran out, the remaining chunks are gone through without any
     for (int64_t c = blockIdx.x; c < args.total_chunks; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
       int pi;
@@ -219,10 +220,10 @@ __global__ void __launch_bounds__(TsmmDmmaKernel<TX, P, Q, CW, STAGES, RS, YS>::
         detail::load_w_frags<TX, K::KS, K::NT>(pr, o0, g, t, b);
         cur = pi;
       }
-      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (ok && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+        ok = false;  // no lane leaves the loop: its MMAs and barriers take the whole warp
         *abort = 1;
         atomicOr(args.error, dev::kErrTimeout);
-        break;
       }
       const int rows = static_cast<int>((pr.rows_main - r0) < RS ? (pr.rows_main - r0) : RS);
       const TX* stage = ring + s * K::STAGE_ALL;

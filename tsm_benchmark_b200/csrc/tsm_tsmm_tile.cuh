@@ -359,6 +359,7 @@ __global__ void __launch_bounds__(kTsmmTileThreads, 1) tsm_tsmm_tile_kernel(cons
     asm volatile("bar.sync 1, %0;" ::"n"(CW * 32) : "memory");
 
     int64_t it = 0;
+    bool ok = true;  // false: a wait ran out, the remaining chunks are gone through without any
     int turn = warp;  // this warp's first unit of the chunk: units go round the warps across chunks
     for (int64_t c = blockIdx.x; c < total; c += G, ++it) {
       const int s = static_cast<int>(it % STAGES);
@@ -373,10 +374,10 @@ __global__ void __launch_bounds__(kTsmmTileThreads, 1) tsm_tsmm_tile_kernel(cons
       const T* x = reinterpret_cast<const T*>(stage);
       T* y = reinterpret_cast<T*>(const_cast<unsigned char*>(stage) + args.y_offset[pi]);
       const double* wf = reinterpret_cast<const double*>(smem + args.w_offset[pi]);
-      if (!dev::mbar_wait_warp(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+      if (ok && !dev::mbar_wait(&full[s], static_cast<uint32_t>((it / STAGES) & 1), abort)) {
+        ok = false;  // no lane leaves the loop: its MMAs and barriers take the whole warp
         *abort = 1;
         atomicOr(args.a.error, dev::kErrTimeout);
-        break;
       }
       if (tsmm_narrow(p, q)) {
         turn = pr.beta ? detail::tsmm_rows<true>(x, y, wf, p, q, rows, turn, lane)
