@@ -296,7 +296,8 @@ bool prefers_tile(const Variant* v, int64_t n, int m, int k, const void* A, int6
 // odd pitch that the columns do not fill) they take four boxes for one: 4 x 4 58
 // -> 75, 8 x 4 57 -> 93, 8 x 8 59 -> 56; within L2 the boxes keep up (60 MB 4 x 4
 // 1.2 times slower, 20 MB as fast, 6 MB 9.9 -> 8.3).  FP32 4 x 8 63 -> 80 stays, with
-// its sums in FP64.  On a
+// its sums in FP64.  A^T A of 5 and 6 columns, boxes of 12 half filled: 300 MB 171
+// -> 228 and 145 -> 191, 60 MB as fast or faster.  On a
 // thousand rows narrow ones cost the same or less direct: 3 x 5 4.8 -> 5.1, FP32 5
 // x 8 4.8 -> 5.7; 13 x 13 7.0 -> 5.5.
 bool pitched_prefers_tile(bool f64, int64_t n, int m, int k, const void* A, int64_t lda, const void* B, int64_t ldb) {
@@ -304,7 +305,8 @@ bool pitched_prefers_tile(bool f64, int64_t n, int m, int k, const void* A, int6
   const int64_t e = f64 ? 8 : 4;
   const int simt_work = padded_width(m) * padded_width(k);  // products a row
   const bool small = m * k < 100 && n < (1 << 14);
-  if (is_gram(m, k, A, lda, B, ldb)) return m >= 5 && !small;  // one load for both operands
+  if (is_gram(m, k, A, lda, B, ldb))  // one load for both operands
+    return m >= 5 && !small && (!f64 || m > 6 || n * m * e < int64_t(128) << 20);
   bool phases = false;
   if (tile_joint(A, m, lda, B, k, ldb, static_cast<size_t>(e), &phases)) {
     if (f64 && phases && simt_work < 64 && n * (m + k) * e >= int64_t(32) << 20) return false;
