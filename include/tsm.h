@@ -202,8 +202,9 @@ tsm_status tsm_gram_f64(tsm_stream_t stream, int64_t n, int m, const double* A, 
  * n <= 2^31 - 8193 (values of r contiguous, columns zero-padded to the
  * kernel's capacity);
  * FP64 tensor cores when the widths rounded up to powers of two multiply to
- * more than 64.  Any other layout (mixed, odd pitches, unaligned) runs on
- * the FP64 tensor cores with each operand loaded its own way.  No
+ * more than 64.  Any other layout (mixed, odd pitches, unaligned, rows that
+ * overlap) runs on the FP64 tensor cores with each operand loaded its own way,
+ * or, for large operands of at most 8 columns, on a direct-load kernel.  No
  * counterpart in the reference, whose operands are always row-major with
  * pitch M (tsmttsm.hh:15-35; sycl_codegen_new.py:66-67).  Same workspace as
  * tsm_gemm_tn_f64 (tsm_gemm_tn_workspace_size(n, m, k)). */

@@ -61,8 +61,8 @@ namespace detail {
 // problems in turn: the product before this one (A^T B in the forward pass or
 // in block orthogonalisation) read A and B in rising row order, and its last
 // reads are what L2 still holds.  B200, rising -> falling order, us: forward and
-// backward of 2^22 x 16 x 16 FP32 264 -> 258, FP64 507 -> 497, of 2^20 x 8 x 8
-// 77 -> 68; block orthogonalisation of 2^20 rows, m = 32, k = 8, 112 -> 100.
+// backward of 2^22 x 16 x 16 FP32 268 -> 265, FP64 502 -> 497, of 2^20 x 8 x 8
+// 76 -> 72; block orthogonalisation of 2^20 rows, m = 32, k = 8, 114 -> 107.
 template <typename T>
 __device__ __forceinline__ void tsmm_chunk(const TsmmArgs<T>& a, int64_t c, int rs, int& pi, int64_t& r0) {
   const int64_t back = a.total_chunks - 1 - c;
