@@ -231,10 +231,10 @@ bool tile_takes(const TsmmProblem<T>& pr) {
 // 118 -> 67, 24 x 24 139 -> 74, 37 x 13 170 -> 75, 48 x 48 219 -> 112, 63 x 63
 // 169 -> 138, 5 x 8 68 -> 69, 1 x 1 297 -> 71, 3 x 3 132 -> 66; FP32 3 x 3 255 ->
 // 77, 24 x 24 269 -> 112, 63 x 63 327 -> 231; 400 MB read, 5 x 8 271 -> 212, 7 x 8 228
-// -> 192.  One FP32 product with 8 columns out of fewer is the exception: the tile
-// kernel writes rows of Y 32 bytes apart to shared memory, where they share banks,
-// the other kernel stores them straight out.  Y = X W, 400
-// MB, 6 x 8 89 -> 103, 7 x 8 83 -> 97, 1 x 8 7 % slower (8 x 7 117 -> 94; at 4 MB as fast).
+// -> 192.  One FP32 product with 8 columns out of fewer is the exception: the
+// tile kernel writes rows of Y 32 bytes apart to shared memory, where they share
+// banks, the other kernel stores them straight out.  Y = X W, 400 MB, 6 x 8 89 ->
+// 103, 7 x 8 83 -> 97, 1 x 8 7 % slower (8 x 7 117 -> 94; at 4 MB as fast).
 // Powers of two, backward: FP64 16 x 16 65 -> 67, 32 x 32 158 -> 178 (500 MB),
 // 64 x 64 113 -> 124, FP32 8 x 8 69 -> 88; on few rows the finer chunks win at
 // 32 and 64, and unequal widths are two launches there: 3 MB of operands, FP64
